@@ -283,10 +283,12 @@ int wbfmm_b200_tree_structure_f(int n, const float *pts, int pstr,
 
 /* M2L kernel selection (all need equal singular and regular orders, else
    the warp kernel runs): 1 (default) = automatic: lane-per-pair kernel up to
-   order 7 (Helmholtz) / 10 (Laplace FP32) / 9 (Laplace FP64), offset-major
-   target tiles above, while their shared memory suffices;
-   2 = lane-per-pair wherever instantiated
-   (Helmholtz <= 8, Laplace <= 16); 3 = target tiles wherever they fit;
+   order 6 (Helmholtz) / 8 (Laplace), matrix products on columns of target
+   boxes above (FP64 on the tensor cores; to order 24 in FP32, 17 / 18 in
+   FP64), offset-major target tiles beyond, while their shared memory
+   suffices; 2 = lane-per-pair wherever instantiated
+   (Helmholtz <= 8, Laplace <= 16); 3 = columns, or target tiles, wherever
+   they fit;
    0 = always the warp-per-target kernel; 4 = Laplace FP32 on the tensor
    cores (dense per-shift operators, tcgen05 kind::tf32 with 3xTF32
    splitting, FP32 accumulation in tensor memory) for equal orders with

@@ -1,0 +1,68 @@
+"""The column M2L kernel against the warp-per-target kernel: local expansions
+at the orders where its tiles change shape (one and two row tiles, 1 to 4 rows
+or 8 and 16 per warp tile, the column counts of its shared-memory plans), on
+dense levels, target lists and sparse storage."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from wbfmm_b200 import engine, workloads as W
+
+pytestmark = pytest.mark.gpu
+
+LAP, HELM = engine.LAPLACE, engine.HELMHOLTZ
+
+
+def _problem(problem, order, depth, n, sphere, k):
+    p = W.serve_request(np.random.default_rng(order), n, problem == HELM, k, sphere)
+    p.depth = depth
+    p.order_s = [0] + [order] * depth
+    p.order_r = list(p.order_s)
+    return p
+
+
+def _locals(p, precision, mode, **kw):
+    cfg = engine.SolverConfig.from_problem(p, precision, **kw)
+    with engine.Solver(cfg) as s:
+        s.set_m2l_kernel(mode)
+        s.set_sources(p.xs).set_strengths(p.q).set_targets(p.xt).run()
+        return [s.coefficients(lv)[1] for lv in range(2, p.depth + 1)], s.field()
+
+
+# tolerances: the two kernels sum the same products in other orders, and a
+# level adds up to 189 translations of about 3 (p + 1) products per value: in
+# FP64 under 1e-13 of the level's norm, in FP32 a few 1e-6
+@pytest.mark.parametrize("precision,tol", [(engine.FP64, 1e-12), (engine.FP32, 2e-5)])
+@pytest.mark.parametrize("problem", [LAP, HELM])
+@pytest.mark.parametrize("order", [2, 3, 4, 7, 8, 10, 11, 12, 14, 15, 16])
+def test_orders(problem, precision, tol, order):
+    p = _problem(problem, order, 3, 3001, False, 18.0)
+    want, _ = _locals(p, precision, 0)
+    got, _ = _locals(p, precision, 3)
+    for a, b in zip(got, want):
+        assert np.linalg.norm(a - b) < tol * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("problem,precision,order", [
+    (HELM, engine.FP64, 17), (LAP, engine.FP64, 18), (HELM, engine.FP32, 19), (HELM, engine.FP32, 20),
+    (HELM, engine.FP32, 24)])
+def test_high_orders(problem, precision, order):
+    p = _problem(problem, order, 2, 1009, False, 25.0)
+    want, _ = _locals(p, precision, 0)
+    got, _ = _locals(p, precision, 3)
+    tol = 1e-12 if precision == engine.FP64 else 2e-5
+    for a, b in zip(got, want):
+        assert np.linalg.norm(a - b) < tol * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("precision,tol", [(engine.FP64, 1e-12), (engine.FP32, 2e-5)])
+@pytest.mark.parametrize("problem", [LAP, HELM])
+@pytest.mark.parametrize("order", [7, 9, 14])
+def test_target_lists_and_sparse(problem, precision, tol, order):
+    p = _problem(problem, order, 4, 5003, True, 30.0)
+    _, (pot, grad) = _locals(p, precision, 0)
+    for kw in (dict(skip_empty=True), dict(sparse=True)):
+        _, (f, g) = _locals(p, precision, 3, **kw)
+        assert np.linalg.norm(f - pot) < tol * np.linalg.norm(pot)
+        assert np.linalg.norm(g - grad) < tol * np.linalg.norm(grad)

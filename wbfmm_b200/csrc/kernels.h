@@ -19,6 +19,8 @@ template <typename T>
 struct OpTables {
   const T* H = nullptr;          // rotation tables, one per theta
   int64_t hstride = 0;
+  const T* HE = nullptr;         // rotation tables in even / odd blocks (m2l_cols.cu)
+  int64_t hestride = 0;
   const int* op_ith = nullptr;   // [kNumOps] theta index
   const int* op_dist = nullptr;  // [kNumOps] list-4 distance index (0..14)
   const T* op_r = nullptr;       // [kNumOps] distance in box widths

@@ -586,10 +586,17 @@ __global__ void k_lanes_reduce(LanesParams<T> p, int N) {
   if (g0 < 0) return;
   const int64_t b = g0 | tau;   // storage index
   T sx = T(0), sy = T(0);
-  for (int s = 0; s < p.nsplit; s++) {
-    T2 v = ((const T2*)p.partial_raw)[(((int64_t)s * 8 + tau) * V + c) * np + plin];
-    sx += v.x; sy += v.y;
+  const T2* part = (const T2*)p.partial_raw + ((int64_t)tau * V + c) * np + plin;
+  const int64_t hop = (int64_t)8 * V * np;
+  int s = 0;
+  for (; s + 8 <= p.nsplit; s += 8) {     // eight loads in flight
+    T2 v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) v[u] = part[(s + u) * hop];
+#pragma unroll
+    for (int u = 0; u < 8; u++) { sx += v[u].x; sy += v[u].y; }
   }
+  for (; s < p.nsplit; s++) { const T2 v = part[s * hop]; sx += v.x; sy += v.y; }
   if (HELM) {
     int64_t o = layout_off(b, c, nc);
     p.cout[2 * o] += sx; p.cout[2 * o + 1] += sy;

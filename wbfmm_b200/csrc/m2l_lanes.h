@@ -95,6 +95,36 @@ int tiles_per_cta(int N, bool* dense = nullptr, bool sparse = false);
 template <typename T>
 int build_helm_coax_rows(const T* raw, int64_t raw_stride, int P, T* out, cudaStream_t s);
 size_t helm_coax_rows_count(int P);
+// matrix products on columns of target boxes (m2l_cols.cu), equal orders up
+// to kColsMaxOrder within the shared-memory limit; sums split over nsplit
+// CTAs per target tile (LanesParams::nsplit from cols_work)
+constexpr int kColsMaxOrder = 24;
+template <typename T, bool HELM>
+bool cols_supported(int Ns, int Nr);
+struct ColsWork {
+  size_t table;   // values of the level's coaxial tables
+  size_t tasks;   // bytes of its warp tiles
+  int nsplit;
+};
+template <typename T, bool HELM>
+ColsWork cols_work(int P, int level);
+// its rotation tables (OpTables::HE) of nth angles from the FP64 ones of
+// degrees <= L: cols_rotation_stride(L) values per angle
+template <typename T>
+int64_t cols_rotation_stride(int L);
+template <typename T>
+int build_cols_rotations(const double* H, int64_t hstride, int nth, int L, T* he, cudaStream_t s);
+// its source rows, (N+1)^2 (Helmholtz complex, Laplace real) per box, of a
+// level array (Layout L), degree n scaled by 2^(scale_e n): lin[tau][row][pp]
+// over the padded parent grid (groups < 0; lanes_lin_bytes), or over the
+// groups stored and a zero column (lanes_lin_groups_bytes)
+template <typename T, bool HELM>
+int cols_planes(const T* arr, int level, int N, int scale_e, int64_t groups, void* lin,
+                cudaStream_t s);
+template <typename T, bool HELM>
+int launch_m2l_cols(const LanesParams<T>& p, const OpTables<T>& t, T* table, void* tasks,
+                    cudaStream_t s);
+
 // smask[sg][padded parent] = the level's box of child type sg under that
 // parent holds sources (0 on the padding), from the level's box counts
 int build_source_mask(const uint32_t* src_n, int level, uint8_t* smask, cudaStream_t s);

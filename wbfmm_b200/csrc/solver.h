@@ -240,6 +240,9 @@ struct Solver : public wbfmm_b200_solver {
   DBuf<uint8_t> smask;              // M2L skip_empty: source boxes of the level holding sources
   DBuf<T> lapsr;                    // Laplace lane M2L: scaled operators of the level
   DBuf<T> hcx;                      // Helmholtz tile M2L: coaxial rows of the level
+  DBuf<T> HE;                       // column M2L: rotation tables in even / odd blocks
+  DBuf<T> cols_cx;                  // and the level's coaxial tables
+  DBuf<unsigned char> cols_tasks;   // and warp tiles
   DBuf<int> flag;
   // outputs (original order)
   DBuf<T> pot, grad;
@@ -320,7 +323,7 @@ struct Solver : public wbfmm_b200_solver {
     f(n32_q); f(n32_dip); f(n32_nx); f(n32_ny); f(n32_nz); f(n32_pot); f(n32_grad);
     f(H64); f(H); f(op_ith); f(op_dist); f(op_r); f(op_ph); f(op_ch);
     for (int i = 0; i < 3; i++) { f(lap64[i]); f(lap[i]); }
-    f(partial); f(lin); f(lanes_part); f(act_scr); f(lapsr); f(hcx); f(smask); f(tc_part);
+    f(partial); f(lin); f(lanes_part); f(act_scr); f(lapsr); f(hcx); f(HE); f(cols_cx); f(cols_tasks); f(smask); f(tc_part);
   }
 
   ~Solver() override {
@@ -715,7 +718,11 @@ struct Solver : public wbfmm_b200_solver {
     WBFMM_TRY(generate_rotation_tables(geom.thetas, L, H64.p, hstride, stream));
     WBFMM_TRY(H.alloc((size_t)hstride * nth));
     WBFMM_TRY(convert_to<T>(H64.p, H.p, (int64_t)hstride * nth, stream));
-    launches += 2;
+    WBFMM_TRY(HE.alloc((size_t)cols_rotation_stride<T>(L) * nth));
+    WBFMM_TRY(build_cols_rotations<T>(H64.p, hstride, nth, L, HE.p, stream));
+    tables.HE = HE.p;
+    tables.hestride = cols_rotation_stride<T>(L);
+    launches += 3;
     if (helm) {
       WBFMM_TRY(helm_coaxial_set());
     } else {
@@ -872,13 +879,19 @@ struct Solver : public wbfmm_b200_solver {
                                : lanes_supported<T, false>(x.Nin, x.Nout);
     const bool tiles_ok = helm ? tiles_supported<T, true>(x.Nin, x.Nout)
                                : tiles_supported<T, false>(x.Nin, x.Nout);
-    // automatic: lanes at the orders where their unrolled code wins, tiles
-    // above, the warp-per-target kernel for what neither covers (Helmholtz
-    // p = 8 runs as fast or faster as tiles in both forms, up to 2x on small
-    // levels, and FP64 Laplace p = 10 15-20% faster, dense or on target
-    // lists; Helmholtz p = 7, FP32 Laplace p = 10 and FP64 Laplace p = 9 run
-    // faster as lanes)
-    const int lanes_max = helm ? 7 : sizeof(T) == 8 ? 9 : 10;
+    // (level 2 of an FP64 Laplace solve keeps the tiles: 8 targets of a type
+    // fill half of its columns' number pairs; 0.121 against 0.110 ms at p = 14)
+    const bool cols_ok = helm ? cols_supported<T, true>(x.Nin, x.Nout)
+                              : cols_supported<T, false>(x.Nin, x.Nout) &&
+                                    !(level == 2 && sizeof(T) == 8);
+    // automatic: lanes at the orders where their unrolled code wins, column
+    // products above (tiles beyond their orders), the warp-per-target kernel
+    // for what none covers.  Lanes / columns, ms on 32768 boxes: Helmholtz
+    // FP32 p = 6 1.37 / 2.90, p = 7 3.32 / 3.32 (4096 boxes 0.61 / 0.47);
+    // FP64 p = 6 4.13 / 5.84, p = 7 11.8 / 8.0; Laplace FP32 p = 8 1.25 / 2.11,
+    // p = 9 3.86 / 2.40; FP64 p = 8 4.11 / 4.42, p = 9 10.4 / 5.3; target lists
+    // change sides at the same orders
+    const int lanes_max = helm ? 6 : 8;
     bool use_tiles = false, use_lanes = false;
     const int he = helm ? helm_e[level] : 0;
     if (cfg.sparse) return m2l_sparse(level, x, he, tiles_ok, lanes_ok, lanes_max);
@@ -899,6 +912,7 @@ struct Solver : public wbfmm_b200_solver {
     } else if (m2l_mode == 3) {
       use_tiles = tiles_ok;
     }
+    if (use_tiles && cols_ok) return m2l_cols(level, x, he);
     if (use_tiles) {
       // offset-major target tiles on the transposed singular expansions
       WBFMM_TRY(lin.alloc(lanes_lin_bytes(level, x.Nin, helm, sizeof(T))));
@@ -1005,6 +1019,50 @@ struct Solver : public wbfmm_b200_solver {
                 : launch_m2l<T, false>(x, tables, stream);
   }
 
+  // The M2L of a level as matrix products on columns of target boxes
+  // (m2l_cols.cu), dense or on sparse storage
+  int m2l_cols(int level, const XlateParams<T>& x, int he) {
+    LanesParams<T> lp;
+    memset(&lp, 0, sizeof(lp));
+    lp.level = level; lp.N = x.Nin;
+    lp.cout = x.cout;
+    lp.coax = x.coax; lp.coax_stride = x.coax_stride;
+    lp.width = x.width; lp.tmask = x.tmask; lp.lap_e = x.lap_e;
+    lp.helm_e = he;
+    const int64_t G = cfg.sparse ? ngroups[level] : -1;
+    WBFMM_TRY(lin.alloc(cfg.sparse ? lanes_lin_groups_bytes(G, x.Nin, helm, sizeof(T))
+                                   : lanes_lin_bytes(level, x.Nin, helm, sizeof(T))));
+    WBFMM_TRY((helm ? cols_planes<T, true>(x.cin, level, x.Nin, he, G, lin.p, stream)
+                    : cols_planes<T, false>(x.cin, level, x.Nin, x.lap_e, G, lin.p, stream)));
+    lp.lin_raw = lin.p;
+    if (cfg.sparse) {
+      WBFMM_TRY(pmap.alloc(source_mask_bytes(level) / 8));
+      WBFMM_TRY(build_parent_slot_map(gmap[level].p, level, (uint32_t)G, pmap.p, stream));
+      lp.pmap = pmap.p; lp.gmap = gmap[level].p; lp.lin_stride = G + 1;
+      launches++;
+    }
+    if (x.tmask) {
+      if (act[level].p) { lp.act = act[level].p; lp.act_n = act_n[level].p; }
+      WBFMM_TRY(smask.alloc(source_mask_bytes(level)));
+      WBFMM_TRY(build_source_mask(x.src_n, level, smask.p, stream));
+      lp.smask = smask.p;
+      launches++;
+    }
+    const ColsWork w = helm ? cols_work<T, true>(x.Nin, level) : cols_work<T, false>(x.Nin, level);
+    WBFMM_TRY(cols_cx.alloc(w.table));
+    WBFMM_TRY(cols_tasks.alloc(w.tasks));
+    lp.nsplit = w.nsplit;
+    if (w.nsplit > 1) {
+      const int V = helm ? (x.Nin + 1) * (x.Nin + 1) : (x.Nin + 1) * (x.Nin + 2) / 2;
+      const int64_t np = (int64_t)1 << (3 * (level - 1));
+      WBFMM_TRY(lanes_part.alloc((size_t)w.nsplit * 8 * V * np * 2));
+      lp.partial_raw = lanes_part.p;
+    }
+    launches += w.nsplit > 1 ? 4 : 3;
+    return helm ? launch_m2l_cols<T, true>(lp, tables, cols_cx.p, cols_tasks.p, stream)
+                : launch_m2l_cols<T, false>(lp, tables, cols_cx.p, cols_tasks.p, stream);
+  }
+
   // The M2L of a level with sparse storage: the lane or tile kernel (the
   // automatic choice, or the one set with set_m2l_kernel 2 / 3) on compact
   // transposed sources, one column per stored source group and a zero
@@ -1020,6 +1078,9 @@ struct Solver : public wbfmm_b200_solver {
     if (!use_lanes && tc == 0) use_lanes = !he && lanes_ok;
     if (!use_lanes && tc == 0)
       return set_error(WBFMM_B200_E_ORDER, "sparse level storage: the M2L needs equal orders in [2, 60] at each level");
+    if (!use_lanes && (helm ? cols_supported<T, true>(x.Nin, x.Nout)
+                            : cols_supported<T, false>(x.Nin, x.Nout)))
+      return m2l_cols(level, x, he);
     const int64_t G = ngroups[level];
     const int se = helm ? he : x.lap_e;
     WBFMM_TRY(lin.alloc(lanes_lin_groups_bytes(G, x.Nin, helm, sizeof(T))));

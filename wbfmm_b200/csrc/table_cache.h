@@ -22,6 +22,7 @@
 #include "engine.h"
 #include "fmm_math.cuh"
 #include "kernels.h"
+#include "m2l_lanes.h"
 #include "tables.h"
 
 namespace wbfmm {
@@ -68,6 +69,7 @@ struct TableCache {
     int64_t hstride = 0;
     int nth = 0;
     double* H64 = nullptr; float* H32 = nullptr;
+    double* HE64 = nullptr; float* HE32 = nullptr;
     int* op_ith = nullptr; int* op_dist = nullptr;
     double* r64 = nullptr; float* r32 = nullptr;
     double* ph64 = nullptr; float* ph32 = nullptr;
@@ -89,7 +91,7 @@ struct TableCache {
   // release every table (no solve may be using them)
   void clear() {
     for (Geo* g : geos) {
-      void* ps[] = {g->H64, g->H32, g->op_ith, g->op_dist, g->r64, g->r32,
+      void* ps[] = {g->H64, g->H32, g->HE64, g->HE32, g->op_ith, g->op_dist, g->r64, g->r32,
                     g->ph64, g->ph32, g->ch64, g->ch32, g->lap64[0], g->lap64[1],
                     g->lap64[2], g->lap32[0], g->lap32[1], g->lap32[2]};
       for (void* p : ps) cudaFree(p);
@@ -129,7 +131,7 @@ struct TableCache {
   // release a Geo's tables and event (stream-ordered on s for pool memory)
   // and the Geo
   void drop_geo(Geo* g, cudaStream_t s) {
-    void* ps[] = {g->H64, g->H32, g->op_ith, g->op_dist, g->r64, g->r32,
+    void* ps[] = {g->H64, g->H32, g->HE64, g->HE32, g->op_ith, g->op_dist, g->r64, g->r32,
                   g->ph64, g->ph32, g->ch64, g->ch32, g->lap64[0], g->lap64[1],
                   g->lap64[2], g->lap32[0], g->lap32[1], g->lap32[2]};
     for (void* p : ps)
@@ -188,6 +190,10 @@ struct TableCache {
     WBFMM_CACHE_TRY(dalloc(g, &g->H32, nh, s));
     WBFMM_CACHE_TRY(generate_rotation_tables(geom.thetas, L, g->H64, g->hstride, s));
     WBFMM_CACHE_TRY(narrow(g->H64, g->H32, (int64_t)nh, s));
+    WBFMM_CACHE_TRY(dalloc(g, &g->HE64, (size_t)cols_rotation_stride<double>(L) * g->nth, s));
+    WBFMM_CACHE_TRY(dalloc(g, &g->HE32, (size_t)cols_rotation_stride<float>(L) * g->nth, s));
+    WBFMM_CACHE_TRY(build_cols_rotations(g->H64, g->hstride, g->nth, L, g->HE64, s));
+    WBFMM_CACHE_TRY(build_cols_rotations(g->H64, g->hstride, g->nth, L, g->HE32, s));
     const size_t n3 = (size_t)(L + 1) * (L + 1) * (L + 1);
     for (int i = 0; i < 3; i++) {
       WBFMM_CACHE_TRY(dalloc(g, &g->lap64[i], n3, s));
@@ -220,6 +226,8 @@ struct TableCache {
     const bool f32 = sizeof(T) == 4;
     t->H = f32 ? (const T*)g->H32 : (const T*)g->H64;
     t->hstride = g->hstride;
+    t->HE = f32 ? (const T*)g->HE32 : (const T*)g->HE64;
+    t->hestride = cols_rotation_stride<T>(g->L);
     t->op_ith = g->op_ith;
     t->op_dist = g->op_dist;
     t->op_r = f32 ? (const T*)g->r32 : (const T*)g->r64;
