@@ -8,6 +8,7 @@
 #include <stddef.h>
 
 #include <atomic>
+#include <mutex>
 #include <vector>
 
 #include "fmm_math.cuh"
@@ -30,21 +31,23 @@ const char* last_error();
 // Raise kernel K's dynamic shared-memory limit on the current device to at
 // least `bytes`, calling the runtime only when a larger size is first needed
 // (cudaFuncSetAttribute takes the driver's locks: issued before every
-// launch it serialised the host threads of concurrent solves).
+// launch it serialised the host threads of concurrent solves).  The calls of
+// a kernel are made one at a time: of two threads raising a limit at once,
+// the smaller size could otherwise be set last and fail the other's launch.
 template <auto K>
 int ensure_smem(size_t bytes) {
   static std::atomic<int> done[64];
+  static std::mutex mu;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
     cudaGetLastError();
     dev = -1;
   }
-  int cur = dev >= 0 ? done[dev].load(std::memory_order_relaxed) : 0;
-  if (dev >= 0 && (int)bytes <= cur) return 0;
+  if (dev >= 0 && (int)bytes <= done[dev].load(std::memory_order_acquire)) return 0;
+  std::lock_guard<std::mutex> lk(mu);
+  if (dev >= 0 && (int)bytes <= done[dev].load(std::memory_order_relaxed)) return 0;
   WBFMM_CUDA(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  if (dev >= 0)
-    while (cur < (int)bytes && !done[dev].compare_exchange_weak(cur, (int)bytes)) {
-    }
+  if (dev >= 0) done[dev].store((int)bytes, std::memory_order_release);
   return 0;
 }
 // WBFMM_SMEM(bytes, kernel): ensure_smem, returning its status on failure
