@@ -287,7 +287,7 @@ int wbfmm_b200_tree_structure_f(int n, const float *pts, int pstr,
    boxes above (FP64 on the tensor cores; to order 24 in FP32, 17 / 18 in
    FP64), offset-major target tiles beyond, while their shared memory
    suffices; 2 = lane-per-pair wherever instantiated
-   (Helmholtz <= 8, Laplace <= 16); 3 = columns, or target tiles, wherever
+   (Helmholtz <= 8, Laplace <= 10), columns elsewhere; 3 = columns, or target tiles, wherever
    they fit;
    0 = always the warp-per-target kernel; 4 = Laplace FP32 on the tensor
    cores (dense per-shift operators, tcgen05 kind::tf32 with 3xTF32

@@ -21,6 +21,8 @@ struct OpTables {
   int64_t hstride = 0;
   const T* HE = nullptr;         // rotation tables in even / odd blocks (m2l_cols.cu)
   int64_t hestride = 0;
+  const T* HL = nullptr;         // and as the lane kernel reads them (m2l_lanes.cu)
+  int64_t hlstride = 0;
   const int* op_ith = nullptr;   // [kNumOps] theta index
   const int* op_dist = nullptr;  // [kNumOps] list-4 distance index (0..14)
   const T* op_r = nullptr;       // [kNumOps] distance in box widths

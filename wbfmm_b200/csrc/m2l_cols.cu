@@ -341,7 +341,8 @@ __global__ void k_cols_rotations(const double* __restrict__ H, int64_t hstride,
 // one (n, m >= 0) of one parent: its eight children are consecutive values.
 template <typename T, bool HELM>
 __global__ void k_cols_planes(const T* __restrict__ arr, int level, int N, int scale_e,
-                              int64_t groups, int64_t ncols, T* __restrict__ lin) {
+                              int64_t groups, int64_t ncols, bool boxmajor,
+                              T* __restrict__ lin) {
   typedef typename P2<T>::t T2;
   const int64_t pp = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (pp >= ncols) return;
@@ -361,6 +362,8 @@ __global__ void k_cols_planes(const T* __restrict__ arr, int level, int N, int s
   }
   const int er = e_row(n, m), orow = m ? o_row(N, n, m) : 0;
   const int se = scale_e * n;
+  // row and column steps of lin, and the type's start
+  const int64_t rs = boxmajor ? 1 : ncols, first = boxmajor ? pp * V : pp;
 #pragma unroll
   for (int tau = 0; tau < 8; tau++) {
     if (HELM) {
@@ -375,14 +378,14 @@ __global__ void k_cols_planes(const T* __restrict__ arr, int level, int N, int s
         }
       }
       const T h = m ? T(0.5) : T(1);
-      T2* o = (T2*)lin + (int64_t)tau * V * ncols + pp;
+      T2* o = (T2*)lin + (int64_t)tau * V * ncols + first;
       T2 s;
       s.x = scale2(h * (a.x + b.x), se); s.y = scale2(h * (a.y + b.y), se);
-      o[(int64_t)er * ncols] = s;
+      o[er * rs] = s;
       if (m) {
         // -i (a - b) / 2
         s.x = scale2(h * (a.y - b.y), se); s.y = -scale2(h * (a.x - b.x), se);
-        o[(int64_t)orow * ncols] = s;
+        o[orow * rs] = s;
       }
     } else {
       T a = T(0), b = T(0);
@@ -390,9 +393,9 @@ __global__ void k_cols_planes(const T* __restrict__ arr, int level, int N, int s
         a = arr[(P * nc + (m ? lidx(n, m) : n * n)) * 8 + tau];
         if (m) b = arr[(P * nc + lidx(n, m) + 1) * 8 + tau];
       }
-      T* o = lin + (int64_t)tau * V * ncols + pp;
-      o[(int64_t)er * ncols] = scale2(a, se);
-      if (m) o[(int64_t)orow * ncols] = scale2(b, se);
+      T* o = lin + (int64_t)tau * V * ncols + first;
+      o[er * rs] = scale2(a, se);
+      if (m) o[orow * rs] = scale2(b, se);
     }
   }
 }
@@ -1160,11 +1163,11 @@ ColsWork cols_work(int P, int level) {
 
 template <typename T, bool HELM>
 int cols_planes(const T* arr, int level, int N, int scale_e, int64_t groups, void* lin,
-                cudaStream_t s) {
+                cudaStream_t s, bool boxmajor) {
   const int64_t npx = (1 << (level - 1)) + 2;
   const int64_t ncols = groups >= 0 ? groups + 1 : npx * npx * npx;
   k_cols_planes<T, HELM><<<dim3((unsigned)((ncols + 127) / 128), o_base(N)), 128, 0, s>>>(
-      arr, level, N, scale_e, groups, ncols, (T*)lin);
+      arr, level, N, scale_e, groups, ncols, boxmajor, (T*)lin);
   WBFMM_CUDA(cudaGetLastError());
   return 0;
 }
@@ -1195,7 +1198,7 @@ int launch_m2l_cols(const LanesParams<T>& p, const OpTables<T>& t, T* table, voi
 #define WBFMM_COLS_INST(T, H)                                                              \
   template bool cols_supported<T, H>(int, int);                                            \
   template ColsWork cols_work<T, H>(int, int);                                             \
-  template int cols_planes<T, H>(const T*, int, int, int, int64_t, void*, cudaStream_t);   \
+  template int cols_planes<T, H>(const T*, int, int, int, int64_t, void*, cudaStream_t, bool); \
   template int launch_m2l_cols<T, H>(const LanesParams<T>&, const OpTables<T>&, T*, void*, \
                                      cudaStream_t);
 WBFMM_COLS_INST(double, true)

@@ -6,11 +6,17 @@
 // with one rotate / coaxial / rotate-back operator.  A CTA takes 128 target
 // parents of one type; its 4 warps x 32 lanes each own one target.  The CTA
 // walks the 189 offsets in a fixed order; for each it stages the offset's
-// operator in shared memory (rotation block H_n^{nu,m}(theta) for n <= P,
-// the phases e^{i m ph}, e^{i m ch}, and the coaxial coefficients), and every
+// operator in shared memory while the lanes apply the one before, and every
 // lane applies it to its own source vector (shared-memory broadcast of the
-// operator, per-lane vectors).  Degree and order loops are unrolled for the
-// compile-time order P, so each lane's inner work is straight-line FMA code.
+// operator, 16 bytes at a time, per-lane vectors).  Degree and order loops
+// are unrolled for the compile-time order P, so each lane's inner work is
+// straight-line FMA code.
+//
+// The vectors are kept in the even / odd basis of m2l_cols.cu (there the
+// derivation): rotation blocks over m, nu >= 0 only, half the products and
+// half the operator reads of the full ones, each coaxial coefficient read
+// once for both parts, and no phases between the rotations.  Laplace's half
+// vectors are that basis already (E the real, O'' the imaginary parts).
 //
 // Sources are read from a transposed copy of the level's singular
 // expansions: per child type, per coefficient, a parent grid padded by one
@@ -18,6 +24,8 @@
 // zeros, exactly the reference's clipping), consecutive lanes reading
 // consecutive parents.
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 #include "engine.h"
 #include "kernels.h"
@@ -175,6 +183,11 @@ __device__ __forceinline__ void cp_async_t(double* dst, const double* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src));
 }
+// 16 bytes, both sides 16-byte aligned
+__device__ __forceinline__ void cp_async_16(void* dst, const void* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src));
+}
 __device__ __forceinline__ void cp_async_commit() {
   asm volatile("cp.async.commit_group;\n" ::);
 }
@@ -182,14 +195,53 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
 
+// Operator tables, rows of a multiple of 16 bytes (lane_pad values): per
+// degree n, rows nu = 0..n of H(nu,m) + H(nu,-m) (H(nu,0) for m = 0) over
+// m = 0..n, then rows nu = 1..n of H(nu,m) - H(nu,-m) over m = 1..n; per
+// order m, rows n = m..P of the coaxial coefficients over l = m..P
+// (Helmholtz: complex).
+template <typename T>
+HD constexpr int lane_pad(int n) {
+  const int v = 16 / (int)sizeof(T);
+  return (n + v - 1) / v * v;
+}
+template <typename T>
+HD constexpr int lane_h(int n) {          // first value of degree n
+  int s = 0;
+  for (int i = 0; i < n; i++) s += (i + 1) * lane_pad<T>(i + 1) + i * lane_pad<T>(i);
+  return s;
+}
+template <typename T, bool HELM>
+HD constexpr int lane_c(int P, int m) {   // and of order m
+  int s = 0;
+  for (int i = 0; i < m; i++) s += (P + 1 - i) * lane_pad<T>((P + 1 - i) * (HELM ? 2 : 1));
+  return s;
+}
+HD constexpr int le_row(int n, int m) { return n * (n + 1) / 2 + m; }
+HD constexpr int lo_row(int P, int n, int m) { return (P + 1) * (P + 2) / 2 + n * (n - 1) / 2 + m - 1; }
+
 template <int P>
 struct LaneDims {
   static constexpr int VF = (P + 1) * (P + 1);                 // full vector
   static constexpr int VH = (P + 1) * (P + 2) / 2;             // half vector
-  static constexpr int NH = (P + 1) * (P + 2) * (4 * P + 3) / 6;  // H, n <= P
-  static constexpr int NC = (P + 1) * (P + 2) * (P + 3) / 6;   // coaxial
-  static constexpr int NL = (P + 1) * (P + 1) * (P + 1);       // Laplace S|R
 };
+
+// n values of a table row (16-byte aligned), as a compile-time array
+template <typename T, int N>
+struct __align__(16) LaneRow {
+  T v[lane_pad<T>(N)];
+};
+template <int N, typename T>
+__device__ __forceinline__ void lane_row(const T* p, LaneRow<T, N>& r) {
+  struct __align__(16) W { T v[16 / sizeof(T)]; };
+  constexpr int VL = 16 / (int)sizeof(T);
+#pragma unroll
+  for (int i = 0; i < lane_pad<T>(N); i += VL) {
+    const W w = *reinterpret_cast<const W*>(p + i);
+#pragma unroll
+    for (int j = 0; j < VL; j++) r.v[i + j] = w.v[j];
+  }
+}
 
 // whether a lane keeps its working vector in registers (about 100 of them at
 // most); otherwise it is a shared-memory column like the accumulator
@@ -235,24 +287,19 @@ struct WVec<T2, V, true> {
   __device__ __forceinline__ T2& operator[](int i) { return r[i]; }
 };
 
-// shared memory layout, in units of T: [H: NH][eph: 2(P+1)][ech: 2(P+1)]
-// [coax: Helmholtz 2 NC | Laplace NL] then per warp the accumulator column
-// and, unless the working vector is in registers, its column; as many
-// warps (<= 4) as fit in 200 KB
+// shared memory layout, in units of T: two operator buffers [H][ech: 2(P+1)]
+// [coax] then per warp the accumulator column and, unless the working vector
+// is in registers, its column; as many warps (<= 4) as fit in 220 KB
 template <typename T, bool HELM, int P>
 struct LaneSmem {
   static constexpr int ncols = LaneReg<T, HELM, P>::value ? 1 : 2;
   static constexpr size_t col_bytes =
       ncols * sizeof(T) * 2 * (size_t)(HELM ? LaneDims<P>::VF : LaneDims<P>::VH) * 32;
-  static constexpr int off_eph = LaneDims<P>::NH;
-  static constexpr int off_ech = off_eph + 2 * (P + 1);
-  static constexpr int off_cx = off_ech + 2 * (P + 1);
-  static constexpr int ops = off_cx + (HELM ? 2 * LaneDims<P>::NC : LaneDims<P>::NL);
-  static constexpr int ops_pad = (ops + 3) & ~3;   // one operator buffer
-  // Laplace stages the next offset's operator while the lanes apply the
-  // current one (two buffers); Helmholtz stages between barriers (one)
-  static constexpr bool DB = !HELM;
-  static constexpr size_t ops_bytes = sizeof(T) * (size_t)((DB ? 2 : 1) * ops_pad);
+  static constexpr int nh = lane_h<T>(P + 1), nc = lane_c<T, HELM>(P, P + 1);
+  static constexpr int off_ech = nh;
+  static constexpr int off_cx = off_ech + lane_pad<T>(2 * (P + 1));
+  static constexpr int ops = off_cx + nc;          // one operator buffer
+  static constexpr size_t ops_bytes = sizeof(T) * (size_t)(2 * ops);
   static constexpr size_t cap = 220 * 1024;
   static constexpr int W = ops_bytes + col_bytes * 4 <= cap ? 4
                          : ops_bytes + col_bytes * 2 <= cap ? 2 : 1;
@@ -262,6 +309,34 @@ struct LaneSmem {
   // per-lane columns (accumulator, working vector) per warp, T2 each
   static constexpr size_t bytes = ops_bytes + col_bytes * W;
 };
+
+// out_i = sum_j row_i[j] in[j] of a table block, out(i, value) called for
+// each i in turn
+template <int ROWS, int N, typename T, typename T2, class Out>
+__device__ __forceinline__ void lane_block(const T* tab, const T2 (&in)[N], Out out) {
+#pragma unroll
+  for (int i = 0; i < ROWS; i++) {
+    LaneRow<T, N> r;
+    lane_row<N>(tab + i * lane_pad<T>(N), r);
+    T2 o;
+    o.x = r.v[0] * in[0].x; o.y = r.v[0] * in[0].y;
+#pragma unroll
+    for (int j = 1; j < N; j++) {
+      o.x = fma(r.v[j], in[j].x, o.x);
+      o.y = fma(r.v[j], in[j].y, o.y);
+    }
+    out(i, o);
+  }
+}
+
+// compile-time loop: f(integral_constant<i>) for i = A..B
+template <int A, int B, class F>
+__device__ __forceinline__ void lane_for(F&& f) {
+  if constexpr (A <= B) {
+    f(std::integral_constant<int, A>());
+    lane_for<A + 1, B>(f);
+  }
+}
 
 template <typename T, bool HELM, int P>
 __global__ void __launch_bounds__(LaneSmem<T, HELM, P>::CTA,
@@ -306,37 +381,24 @@ k_m2l_lanes(LanesParams<T> p, OpTables<T> t) {
 #pragma unroll 1
   for (int c = 0; c < V; c++) { T2 z; z.x = T(0); z.y = T(0); acc[c * 32] = z; }
 
-  // Staging of an offset's operator: the rotation block, both phase sets
-  // and the coaxial coefficients (Helmholtz: the level's table of the
-  // offset's distance; Laplace: the level's scaled S|R of the shift code).
-  // Laplace double-buffers it: while the lanes apply offset j's operator
-  // from one buffer, offset j + nsplit's streams into the other (cp.async),
-  // so one barrier per offset both publishes a buffer and retires the other.
-  auto copy = [&](T* d, const T* src) {
-    if constexpr (SM::DB) cp_async_t(d, src); else *d = *src;
-  };
+  // An offset's operator (rotation block, source and target phases, the
+  // coaxial table of its distance) streams into one buffer by cp.async while
+  // the lanes apply the offset before from the other: one barrier per offset
+  // both publishes a buffer and retires the other.
   auto stage = [&](int j, T* dst) {
     const int op = c_offsets[tau][j] & 511;
-    const T* H = t.H + (int64_t)t.op_ith[op] * t.hstride;
-    for (int i = threadIdx.x; i < LaneDims<P>::NH; i += kLanesCTA) copy(dst + i, H + i);
-    const T* eph = t.ph + (size_t)op * (t.lmax + 1) * 2;
+    constexpr int VL = 16 / (int)sizeof(T);
+    const T* H = t.HL + (int64_t)t.op_ith[op] * t.hlstride;
+    for (int i = threadIdx.x * VL; i < SM::nh; i += kLanesCTA * VL) cp_async_16(dst + i, H + i);
     const T* ech = t.ch + (size_t)op * (t.lmax + 1) * 2;
-    for (int i = threadIdx.x; i < 2 * (P + 1); i += kLanesCTA) {
-      copy(dst + SM::off_eph + i, eph + i);
-      copy(dst + SM::off_ech + i, ech + i);
-    }
-    if (HELM) {
-      const T* cx = p.coax + (int64_t)t.op_dist[op] * p.coax_stride;
-      for (int i = threadIdx.x; i < 2 * LaneDims<P>::NC; i += kLanesCTA)
-        copy(dst + SM::off_cx + i, cx + i);
-    } else {
-      const T* cx = (const T*)p.lapsr + (int64_t)op * LaneDims<P>::NL;
-      for (int i = threadIdx.x; i < LaneDims<P>::NL; i += kLanesCTA)
-        copy(dst + SM::off_cx + i, cx + i);
-    }
-    if constexpr (SM::DB) cp_async_commit();
+    for (int i = threadIdx.x; i < 2 * (P + 1); i += kLanesCTA)
+      cp_async_t(dst + SM::off_ech + i, ech + i);
+    const T* cx = (const T*)p.lanes_cx + (int64_t)t.op_dist[op] * SM::nc;
+    for (int i = threadIdx.x * VL; i < SM::nc; i += kLanesCTA * VL)
+      cp_async_16(dst + SM::off_cx + i, cx + i);
+    cp_async_commit();
   };
-  if (SM::DB && split < 189) stage(split, opsb);
+  if (split < 189) stage(split, opsb);
   int buf = 0;
 #pragma unroll 1
   for (int j = split; j < 189; j += p.nsplit) {
@@ -344,19 +406,11 @@ k_m2l_lanes(LanesParams<T> p, OpTables<T> t) {
     const int sg = (code >> 9) & 7;
     const int ddx = ((code >> 12) & 3) - 1, ddy = ((code >> 14) & 3) - 1,
               ddz = ((code >> 16) & 3) - 1;
-    if constexpr (SM::DB) {
-      cp_async_wait_all();
-      __syncthreads();   // this offset's operator visible; the other buffer free
-      if (j + p.nsplit < 189) stage(j + p.nsplit, opsb + (buf ^ 1) * SM::ops_pad);
-    } else {
-      __syncthreads();   // previous operator no longer in use
-      stage(j, opsb);
-      __syncthreads();
-    }
-    const T* ops = opsb + buf * SM::ops_pad;
-    if constexpr (SM::DB) buf ^= 1;
-    const T* sH = ops;
-    const T* seph = ops + SM::off_eph;
+    cp_async_wait_all();
+    __syncthreads();   // this offset's operator visible; the other buffer free
+    if (j + p.nsplit < 189) stage(j + p.nsplit, opsb + (buf ^ 1) * SM::ops);
+    const T* ops = opsb + buf * SM::ops;
+    buf ^= 1;
     const T* sech = ops + SM::off_ech;
     const T* scx = ops + SM::off_cx;
     if (!active) continue;
@@ -369,92 +423,99 @@ k_m2l_lanes(LanesParams<T> p, OpTables<T> t) {
     const int64_t col = p.pmap ? (int64_t)p.pmap[spp] : spp;
     const int64_t cs = p.boxmajor ? 1 : lstride;
     const T2* src = (const T2*)p.lin_raw + (int64_t)sg * V * lstride + (p.boxmajor ? col * V : col);
-    if (HELM) {
-      // stage A: copy the source into the lane's column with e^{i m ch}
+    if constexpr (HELM) {
+      // source phases: E = c S+ - s S'', O'' = c S'' + s S+
 #pragma unroll
       for (int n = 0; n <= P; n++) {
+        w[le_row(n, 0)] = __ldg(src + (int64_t)le_row(n, 0) * cs);
 #pragma unroll
-        for (int m = -n; m <= n; m++) {
-          const int am = m < 0 ? -m : m;
-          T2 v = __ldg(src + (int64_t)cidx(n, m) * cs);
-          w[cidx(n, m)] = cm(v, sech[2 * am], m < 0 ? -sech[2 * am + 1] : sech[2 * am + 1]);
+        for (int m = 1; m <= n; m++) {
+          const T2 e = __ldg(src + (int64_t)le_row(n, m) * cs);
+          const T2 o = __ldg(src + (int64_t)lo_row(P, n, m) * cs);
+          const T c = sech[2 * m], sn = sech[2 * m + 1];
+          T2 x, y;
+          x.x = c * e.x - sn * o.x; x.y = c * e.y - sn * o.y;
+          y.x = c * o.x + sn * e.x; y.y = c * o.y + sn * e.y;
+          w[le_row(n, m)] = x;
+          w[lo_row(P, n, m)] = y;
         }
         cfence();
       }
-      // stage B: forward rotation per degree, in place, then e^{-i nu ph}
+      // forward rotation per degree, in place
+      lane_for<0, P>([&](auto nn) {
+        constexpr int n = decltype(nn)::value;
+        T2 in[n + 1];
 #pragma unroll
-      for (int n = 0; n <= P; n++) {
-        T2 in[2 * P + 1];
+        for (int m = 0; m <= n; m++) in[m] = w[le_row(n, m)];
+        lane_block<n + 1, n + 1>(ops + lane_h<T>(n), in, [&](int i, T2 v) { w[le_row(n, i)] = v; });
+        if constexpr (n > 0) {
+          T2 io[n];
 #pragma unroll
-        for (int m = -n; m <= n; m++) in[m + n] = w[cidx(n, m)];
-        const int hb = rot_idx(-n, 0, n);
+          for (int m = 0; m < n; m++) io[m] = w[lo_row(P, n, m + 1)];
+          lane_block<n, n>(ops + lane_h<T>(n) + (n + 1) * lane_pad<T>(n + 1), io,
+                           [&](int i, T2 v) { w[lo_row(P, n, i + 1)] = v; });
+        }
+        cfence();
+      });
+      // coaxial (S|R) per order, both parts with one read of the table
+      lane_for<0, P>([&](auto mm) {
+        constexpr int m = decltype(mm)::value, L = P + 1 - m, RS = lane_pad<T>(2 * L);
+        T2 te[L], to[m > 0 ? L : 1];
 #pragma unroll
-        for (int nu = -n; nu <= n; nu++) {
-          T sr = T(0), si = T(0);
+        for (int l = 0; l < L; l++) {
+          te[l] = w[le_row(m + l, m)];
+          if (m > 0) to[l] = w[lo_row(P, m + l, m)];
+        }
 #pragma unroll
-          for (int m = -n; m <= n; m++) {
-            const T h = m >= 0 ? sH[hb + (nu + n) * (n + 1) + m]
-                               : sH[hb + (-nu + n) * (n + 1) - m];
-            sr += h * in[m + n].x;
-            si += h * in[m + n].y;
+        for (int n = 0; n < L; n++) {
+          LaneRow<T, 2 * L> r;
+          lane_row<2 * L>(scx + lane_c<T, true>(P, m) + n * RS, r);
+          T2 a, b;
+          a.x = a.y = b.x = b.y = T(0);
+#pragma unroll
+          for (int l = 0; l < L; l++) {
+            const T cr = r.v[2 * l], ci = r.v[2 * l + 1];
+            a.x += cr * te[l].x - ci * te[l].y;
+            a.y += ci * te[l].x + cr * te[l].y;
+            if (m > 0) {
+              b.x += cr * to[l].x - ci * to[l].y;
+              b.y += ci * to[l].x + cr * to[l].y;
+            }
           }
-          const int an = nu < 0 ? -nu : nu;
-          T2 o; o.x = sr; o.y = si;
-          w[cidx(n, nu)] = cm(o, seph[2 * an], nu < 0 ? seph[2 * an + 1] : -seph[2 * an + 1]);
+          w[le_row(m + n, m)] = a;
+          if (m > 0) w[lo_row(P, m + n, m)] = b;
         }
         cfence();
-      }
-      // stage C: coaxial (S|R) per order m, in place, then e^{i m ph}
+      });
+      // back rotation and target phases: T+ += c E + s O'', T'' += c O'' - s E
+      lane_for<0, P>([&](auto nn) {
+        constexpr int n = decltype(nn)::value;
+        T2 in[n + 1], e[n + 1];
 #pragma unroll
-      for (int m = -P; m <= P; m++) {
-        const int am = m < 0 ? -m : m;
-        T2 tv[P + 1];
+        for (int m = 0; m <= n; m++) in[m] = w[le_row(n, m)];
+        lane_block<n + 1, n + 1>(ops + lane_h<T>(n), in, [&](int i, T2 v) { e[i] = v; });
+        T2 a = acc[le_row(n, 0) * 32];
+        a.x += e[0].x; a.y += e[0].y;
+        acc[le_row(n, 0) * 32] = a;
+        if constexpr (n > 0) {
+          T2 io[n];
 #pragma unroll
-        for (int l = am; l <= P; l++) tv[l] = w[cidx(l, m)];
-#pragma unroll
-        for (int n = am; n <= P; n++) {
-          T sr = T(0), si = T(0);
-#pragma unroll
-          for (int l = am; l <= P; l++) {
-            const int ic = l >= n ? coax_idx(l, am, n) : coax_idx(n, am, l);
-            const T sgn = (l >= n || ((n + l) & 1) == 0) ? T(1) : T(-1);
-            const T cr = sgn * scx[2 * ic], ci = sgn * scx[2 * ic + 1];
-            sr += cr * tv[l].x - ci * tv[l].y;
-            si += ci * tv[l].x + cr * tv[l].y;
-          }
-          T2 o; o.x = sr; o.y = si;
-          w[cidx(n, m)] = cm(o, seph[2 * am], m < 0 ? -seph[2 * am + 1] : seph[2 * am + 1]);
+          for (int m = 0; m < n; m++) io[m] = w[lo_row(P, n, m + 1)];
+          lane_block<n, n>(ops + lane_h<T>(n) + (n + 1) * lane_pad<T>(n + 1), io, [&](int i, T2 o) {
+            const int nu = i + 1;
+            const T c = sech[2 * nu], sn = sech[2 * nu + 1];
+            T2 u = acc[le_row(n, nu) * 32], v = acc[lo_row(P, n, nu) * 32];
+            u.x += c * e[nu].x + sn * o.x; u.y += c * e[nu].y + sn * o.y;
+            v.x += c * o.x - sn * e[nu].x; v.y += c * o.y - sn * e[nu].y;
+            acc[le_row(n, nu) * 32] = u;
+            acc[lo_row(P, n, nu) * 32] = v;
+          });
         }
         cfence();
-      }
-      // stage D: back rotation, acc[n,nu] += e^{-i nu ch} sum_m H w[n,m]
-#pragma unroll
-      for (int n = 0; n <= P; n++) {
-        T2 in[2 * P + 1];
-#pragma unroll
-        for (int m = -n; m <= n; m++) in[m + n] = w[cidx(n, m)];
-        const int hb = rot_idx(-n, 0, n);
-#pragma unroll
-        for (int nu = -n; nu <= n; nu++) {
-          T sr = T(0), si = T(0);
-#pragma unroll
-          for (int m = -n; m <= n; m++) {
-            const T h = m >= 0 ? sH[hb + (nu + n) * (n + 1) + m]
-                               : sH[hb + (-nu + n) * (n + 1) - m];
-            sr += h * in[m + n].x;
-            si += h * in[m + n].y;
-          }
-          const int an = nu < 0 ? -nu : nu;
-          T2 o; o.x = sr; o.y = si;
-          o = cm(o, sech[2 * an], nu < 0 ? sech[2 * an + 1] : -sech[2 * an + 1]);
-          T2 a = acc[cidx(n, nu) * 32];
-          a.x += o.x; a.y += o.y;
-          acc[cidx(n, nu) * 32] = a;
-        }
-        cfence();
-      }
+      });
     } else {
-      // Laplace, half vectors (m >= 0; negative m are conjugates)
+      // Laplace, half vectors (m >= 0; negative m are conjugates): x the even
+      // parts, y the odd ones
 #pragma unroll
       for (int n = 0; n <= P; n++) {
 #pragma unroll
@@ -464,74 +525,60 @@ k_m2l_lanes(LanesParams<T> p, OpTables<T> t) {
         }
         cfence();
       }
-#pragma unroll
-      for (int n = 0; n <= P; n++) {
-        T2 in[P + 1];
+      // (E, O'') of row nu from the degree's vector
+      auto rotate = [&](auto nn, auto out) {
+        constexpr int n = decltype(nn)::value, RE = lane_pad<T>(n + 1), RO = lane_pad<T>(n > 0 ? n : 1);
+        const T* te = ops + lane_h<T>(n);
+        const T* to = te + (n + 1) * RE;
+        T2 in[n + 1];
 #pragma unroll
         for (int m = 0; m <= n; m++) in[m] = w[hidx(n, m)];
-        const int hb = rot_idx(-n, 0, n);
 #pragma unroll
         for (int nu = 0; nu <= n; nu++) {
-          T tr = sH[hb + (nu + n) * (n + 1)] * in[0].x, ti = T(0);
-#pragma unroll
-          for (int m = 1; m <= n; m++) {
-            const T hp = sH[hb + (nu + n) * (n + 1) + m];
-            const T hm = sH[hb + (-nu + n) * (n + 1) + m];
-            tr += (hp + hm) * in[m].x;
-            ti += (hp - hm) * in[m].y;
-          }
-          const T er = seph[2 * nu], ei = seph[2 * nu + 1];
+          LaneRow<T, n + 1> re;
+          lane_row<n + 1>(te + nu * RE, re);
           T2 o;
-          o.x = er * tr + ei * ti;
-          o.y = nu == 0 ? T(0) : er * ti - ei * tr;
-          w[hidx(n, nu)] = o;
+          o.x = re.v[0] * in[0].x; o.y = T(0);
+#pragma unroll
+          for (int m = 1; m <= n; m++) o.x = fma(re.v[m], in[m].x, o.x);
+          if constexpr (n > 0) {
+            if (nu > 0) {
+              LaneRow<T, n> ro;
+              lane_row<n>(to + (nu - 1) * RO, ro);
+#pragma unroll
+              for (int m = 1; m <= n; m++) o.y = fma(ro.v[m - 1], in[m].y, o.y);
+            }
+          }
+          out(nu, o);
         }
         cfence();
-      }
+      };
+      lane_for<0, P>([&](auto nn) {
+        constexpr int n = decltype(nn)::value;
+        rotate(nn, [&](int nu, T2 o) { w[hidx(n, nu)] = o; });
+      });
+      lane_for<0, P>([&](auto mm) {
+        constexpr int m = decltype(mm)::value, L = P + 1 - m, RS = lane_pad<T>(L);
+        T2 tv[L];
 #pragma unroll
-      for (int m = 0; m <= P; m++) {
-        T2 tv[P + 1];
-#pragma unroll
-        for (int nd = m; nd <= P; nd++) tv[nd] = w[hidx(nd, m)];
-#pragma unroll
-        for (int n = m; n <= P; n++) {
-          T sr = T(0), si = T(0);
-#pragma unroll
-          for (int nd = m; nd <= P; nd++) {
-            const T c = scx[(n * (P + 1) + nd) * (P + 1) + m];
-            sr += c * tv[nd].x;
-            si += c * tv[nd].y;
-          }
-          if (m == 0) si = T(0);
-          T2 o; o.x = sr; o.y = si;
-          w[hidx(n, m)] = cm(o, seph[2 * m], seph[2 * m + 1]);
-        }
+        for (int l = 0; l < L; l++) tv[l] = w[hidx(m + l, m)];
+        lane_block<L, L>(scx + lane_c<T, false>(P, m), tv, [&](int i, T2 v) {
+          if (m == 0) v.y = T(0);
+          w[hidx(m + i, m)] = v;
+        });
+        (void)RS;
         cfence();
-      }
-#pragma unroll
-      for (int n = 0; n <= P; n++) {
-        T2 in[P + 1];
-#pragma unroll
-        for (int m = 0; m <= n; m++) in[m] = w[hidx(n, m)];
-        const int hb = rot_idx(-n, 0, n);
-#pragma unroll
-        for (int nu = 0; nu <= n; nu++) {
-          T tr = sH[hb + (nu + n) * (n + 1)] * in[0].x, ti = T(0);
-#pragma unroll
-          for (int m = 1; m <= n; m++) {
-            const T hp = sH[hb + (nu + n) * (n + 1) + m];
-            const T hm = sH[hb + (-nu + n) * (n + 1) + m];
-            tr += (hp + hm) * in[m].x;
-            ti += (hp - hm) * in[m].y;
-          }
+      });
+      lane_for<0, P>([&](auto nn) {
+        constexpr int n = decltype(nn)::value;
+        rotate(nn, [&](int nu, T2 o) {
           const T er = sech[2 * nu], ei = sech[2 * nu + 1];
           T2 a = acc[hidx(n, nu) * 32];
-          a.x += er * tr + ei * ti;
-          if (nu != 0) a.y += er * ti - ei * tr;
+          a.x += er * o.x + ei * o.y;
+          if (nu != 0) a.y += er * o.y - ei * o.x;
           acc[hidx(n, nu) * 32] = a;
-        }
-        cfence();
-      }
+        });
+      });
     }
   }
   if (!active) return;
@@ -539,30 +586,41 @@ k_m2l_lanes(LanesParams<T> p, OpTables<T> t) {
   const int64_t g0 = compact_box(p.gmap, pmort << 3);   // storage index of the group
   if (g0 < 0) return;   // (targets lie in stored groups)
   const int64_t b = g0 | tau;
-  if (p.nsplit == 1) {
-    if (HELM) {
-      for (int c = 0; c < V; c++) {
-        T2 a = acc[c * 32];
-        int64_t o = layout_off(b, c, nc);
-        p.cout[2 * o] += a.x;
-        p.cout[2 * o + 1] += a.y;
-      }
-    } else {
-      for (int c = 0; c < V; c++) {
-        T2 a = acc[c * 32];
-        int n = half_degree(c), m = c - n * (n + 1) / 2;
-        if (m == 0) {
-          p.cout[layout_off(b, n * n, nc)] += a.x;
-        } else {
-          int id = lidx(n, m);
-          p.cout[layout_off(b, id, nc)] += a.x;
-          p.cout[layout_off(b, id + 1, nc)] += a.y;
-        }
+  T2* part = p.nsplit > 1
+                 ? (T2*)p.partial_raw + ((int64_t)split * 8 + tau) * V * np + plin : nullptr;
+  if (HELM) {
+    // (n, +-m) from the even and odd sums: T+ +- i T''
+    auto put = [&](int c, T2 a) {
+      if (part) { part[(int64_t)c * np] = a; return; }
+      const int64_t o = layout_off(b, c, nc);
+      p.cout[2 * o] += a.x;
+      p.cout[2 * o + 1] += a.y;
+    };
+    for (int n = 0; n <= P; n++) {
+      put(cidx(n, 0), acc[le_row(n, 0) * 32]);
+      for (int m = 1; m <= n; m++) {
+        const T2 e = acc[le_row(n, m) * 32], o = acc[lo_row(P, n, m) * 32];
+        T2 u, v;
+        u.x = e.x - o.y; u.y = e.y + o.x;
+        v.x = e.x + o.y; v.y = e.y - o.x;
+        put(cidx(n, m), u);
+        put(cidx(n, -m), v);
       }
     }
-  } else {
-    T2* part = (T2*)p.partial_raw + ((int64_t)split * 8 + tau) * V * np + plin;
+  } else if (part) {
     for (int c = 0; c < V; c++) part[(int64_t)c * np] = acc[c * 32];
+  } else {
+    for (int c = 0; c < V; c++) {
+      T2 a = acc[c * 32];
+      int n = half_degree(c), m = c - n * (n + 1) / 2;
+      if (m == 0) {
+        p.cout[layout_off(b, n * n, nc)] += a.x;
+      } else {
+        int id = lidx(n, m);
+        p.cout[layout_off(b, id, nc)] += a.x;
+        p.cout[layout_off(b, id + 1, nc)] += a.y;
+      }
+    }
   }
 }
 
@@ -610,6 +668,79 @@ __global__ void k_lanes_reduce(LanesParams<T> p, int N) {
       p.cout[layout_off(b, id + 1, nc)] += sy;
     }
   }
+}
+
+// ----------------------------------------------------- operator tables
+template <typename T>
+__global__ void k_lane_rotations(const double* __restrict__ H, int64_t hstride,
+                                 T* __restrict__ out, int64_t stride) {
+  const int n = blockIdx.y, re = lane_pad<T>(n + 1), ro = lane_pad<T>(n);
+  const double* h = H + (int64_t)blockIdx.x * hstride;
+  T* o = out + (int64_t)blockIdx.x * stride + lane_h<T>(n);
+  const int ne = (n + 1) * re;
+  for (int e = threadIdx.x; e < ne + n * ro; e += blockDim.x) {
+    const bool odd = e >= ne;
+    const int i = odd ? e - ne : e, r = odd ? ro : re;
+    const int nu = i / r + (odd ? 1 : 0), m = i % r + (odd ? 1 : 0);
+    double v = 0.0;
+    if (m <= n) {
+      const double a = h[rot_idx(nu, m, n)], b = h[rot_idx(-nu, m, n)];
+      v = odd ? a - b : m ? a + b : a;
+    }
+    o[e] = (T)v;
+  }
+}
+__constant__ int c_lane_dist2[15] = {4, 5, 6, 8, 9, 10, 11, 12, 13, 14, 17, 18, 19, 22, 27};
+// block (distance, order)
+template <typename T, bool HELM>
+__global__ void k_lane_coax(LanesParams<T> p, OpTables<T> t, T* __restrict__ out) {
+  const int P = p.N, d = blockIdx.x, m = blockIdx.y, L = P + 1 - m;
+  const int rs = lane_pad<T>(L * (HELM ? 2 : 1));
+  T* o = out + (int64_t)d * lane_c<T, HELM>(P, P + 1) + lane_c<T, HELM>(P, m);
+  for (int e = threadIdx.x; e < L * rs; e += blockDim.x) {
+    const int n = m + e / rs, j = e % rs, l = m + (HELM ? j / 2 : j);
+    T v = T(0);
+    if (l <= P) {
+      if (HELM) {
+        const T* c = p.coax + (int64_t)d * p.coax_stride;
+        const int ic = l >= n ? coax_idx(l, m, n) : coax_idx(n, m, l);
+        const T sg = (l >= n || ((n + l) & 1) == 0) ? T(1) : T(-1);
+        v = sg * c[2 * ic + (j & 1)];
+      } else {
+        // S|R(n, l, m) / (r^(n+1) (2^e r)^l) on sources scaled by 2^(e l)
+        const T r = p.width * (T)sqrt((double)c_lane_dist2[d]);
+        const T rinv = T(1) / r, qinv = T(1) / scale2(r, p.lap_e);
+        T sc = rinv, q = T(1);
+        for (int k = 0; k < n; k++) sc *= rinv;
+        for (int k = 0; k < l; k++) q *= qinv;
+        const int D = t.lt + 1;
+        v = (t.lapSR[((int64_t)n * D + l) * D + m] * q) * sc;
+      }
+    }
+    o[e] = v;
+  }
+}
+static int lane_degrees(int L) { return L < kLanesMaxLap ? L : kLanesMaxLap; }
+template <typename T>
+int64_t lane_rotation_stride(int L) { return lane_h<T>(lane_degrees(L) + 1); }
+template int64_t lane_rotation_stride<float>(int);
+template int64_t lane_rotation_stride<double>(int);
+template <typename T>
+int build_lane_rotations(const double* H, int64_t hstride, int nth, int L, T* out, cudaStream_t s) {
+  k_lane_rotations<T><<<dim3(nth, lane_degrees(L) + 1), 128, 0, s>>>(H, hstride, out,
+                                                                     lane_rotation_stride<T>(L));
+  WBFMM_CUDA(cudaGetLastError());
+  return 0;
+}
+template int build_lane_rotations<float>(const double*, int64_t, int, int, float*, cudaStream_t);
+template int build_lane_rotations<double>(const double*, int64_t, int, int, double*, cudaStream_t);
+template <typename T, bool HELM>
+size_t lane_coax_count(int P) { return (size_t)15 * lane_c<T, HELM>(P, P + 1); }
+template <typename T, bool HELM>
+int build_lane_coax(const LanesParams<T>& p, const OpTables<T>& t, T* out, cudaStream_t s) {
+  k_lane_coax<T, HELM><<<dim3(15, p.N + 1), 128, 0, s>>>(p, t, out);
+  WBFMM_CUDA(cudaGetLastError());
+  return 0;
 }
 
 // ------------------------------------------------- Laplace operators
@@ -828,8 +959,7 @@ bool lanes_supported(int Ns, int Nr) {
   case PP: return LaneSmem<T, HELM, PP>::fits;
     WBFMM_LANES_FIT(2) WBFMM_LANES_FIT(3) WBFMM_LANES_FIT(4) WBFMM_LANES_FIT(5)
     WBFMM_LANES_FIT(6) WBFMM_LANES_FIT(7) WBFMM_LANES_FIT(8) WBFMM_LANES_FIT(9)
-    WBFMM_LANES_FIT(10) WBFMM_LANES_FIT(11) WBFMM_LANES_FIT(12) WBFMM_LANES_FIT(13)
-    WBFMM_LANES_FIT(14) WBFMM_LANES_FIT(15) WBFMM_LANES_FIT(16)
+    WBFMM_LANES_FIT(10)
 #undef WBFMM_LANES_FIT
     default: return false;
   }
@@ -861,12 +991,6 @@ int launch_m2l_lanes(const LanesParams<T>& p, const OpTables<T>& t,
   case PP: return launch_lanes_P<T, false, PP>(p, t, s);
       WBFMM_LANES_CASE(9)
       WBFMM_LANES_CASE(10)
-      WBFMM_LANES_CASE(11)
-      WBFMM_LANES_CASE(12)
-      WBFMM_LANES_CASE(13)
-      WBFMM_LANES_CASE(14)
-      WBFMM_LANES_CASE(15)
-      WBFMM_LANES_CASE(16)
 #undef WBFMM_LANES_CASE
       default: break;
     }
@@ -875,6 +999,8 @@ int launch_m2l_lanes(const LanesParams<T>& p, const OpTables<T>& t,
 }
 
 #define WBFMM_LANES_INST(T, H)                                                   \
+  template size_t lane_coax_count<T, H>(int);                                    \
+  template int build_lane_coax<T, H>(const LanesParams<T>&, const OpTables<T>&, T*, cudaStream_t); \
   template int lanes_to_lin<T, H>(const T*, int, int, int, void*, cudaStream_t, bool); \
   template int lanes_to_lin_groups<T, H>(const T*, int64_t, int, int, void*, cudaStream_t, bool); \
   template int launch_lanes_reduce<T, H>(const LanesParams<T>&, cudaStream_t);   \

@@ -9,7 +9,7 @@
 namespace wbfmm {
 
 constexpr int kLanesMaxHelm = 8;    // orders instantiated for Helmholtz
-constexpr int kLanesMaxLap = 16;    // and for Laplace
+constexpr int kLanesMaxLap = 10;    // and for Laplace
 
 template <typename T>
 struct LanesParams {
@@ -26,7 +26,8 @@ struct LanesParams {
   int helm_e;           // Helmholtz tiles (helm_m2l_exp): degree l of lin_raw is
                         // scaled by 2^(helm_e l), coax by 2^(-helm_e (n + l)),
                         // and output degree n by 2^(helm_e n)
-  const void* lapsr;    // Laplace: [kNumOps][(P+1)^3] scaled S|R per shift (build_lap_sr_ops)
+  const void* lapsr;    // Laplace tiles: [kNumOps][(P+1)^3] scaled S|R per shift (build_lap_sr_ops)
+  const void* lanes_cx; // lane kernel: the level's coaxial tables (build_lane_coax)
   const void* hcx;      // Helmholtz tiles: the level's coaxial rows (build_helm_coax_rows)
   const int* act;       // sparse targets: [8][np] parents per child type, or null
   const int* act_n;     // [8] list lengths (device)
@@ -73,6 +74,18 @@ inline void build_offset_table(int* tab) {
 
 template <typename T, bool HELM>
 bool lanes_supported(int Ns, int Nr);
+// The lane kernel's tables: rotations (OpTables::HL) of nth angles from the
+// FP64 ones, in even / odd blocks of degrees <= L, lane_rotation_stride(L)
+// values per angle; a level's coaxial tables of the 15 distances,
+// lane_coax_count(P) values in all
+template <typename T>
+int64_t lane_rotation_stride(int L);
+template <typename T>
+int build_lane_rotations(const double* H, int64_t hstride, int nth, int L, T* out, cudaStream_t s);
+template <typename T, bool HELM>
+size_t lane_coax_count(int P);
+template <typename T, bool HELM>
+int build_lane_coax(const LanesParams<T>& p, const OpTables<T>& t, T* out, cudaStream_t s);
 // sum of the split partial results (split order) into the level array
 template <typename T, bool HELM>
 int launch_lanes_reduce(const LanesParams<T>& p, cudaStream_t s);
@@ -117,10 +130,11 @@ int build_cols_rotations(const double* H, int64_t hstride, int nth, int L, T* he
 // its source rows, (N+1)^2 (Helmholtz complex, Laplace real) per box, of a
 // level array (Layout L), degree n scaled by 2^(scale_e n): lin[tau][row][pp]
 // over the padded parent grid (groups < 0; lanes_lin_bytes), or over the
-// groups stored and a zero column (lanes_lin_groups_bytes)
+// groups stored and a zero column (lanes_lin_groups_bytes); boxmajor:
+// lin[tau][pp][row]
 template <typename T, bool HELM>
 int cols_planes(const T* arr, int level, int N, int scale_e, int64_t groups, void* lin,
-                cudaStream_t s);
+                cudaStream_t s, bool boxmajor = false);
 template <typename T, bool HELM>
 int launch_m2l_cols(const LanesParams<T>& p, const OpTables<T>& t, T* table, void* tasks,
                     cudaStream_t s);
@@ -154,7 +168,7 @@ int build_parent_slot_map(const uint32_t* gmap, int level, uint32_t groups, uint
 // act_n[8].  act holds 8^level ints; scratch active_list_scratch(level) ints.
 size_t active_list_scratch(int level);
 
-// Laplace M2L operators of one level for the lane kernel, per shift code:
+// Laplace M2L operators of one level for the tile kernel, per shift code:
 // out[op][(n (P+1) + nd) (P+1) + m] = S|R(n, nd, m) / (t^(n+1) (2^e t)^nd),
 // t = width |d_op| (the scaled form of lap_scale_exp)
 template <typename T>

@@ -238,10 +238,11 @@ struct Solver : public wbfmm_b200_solver {
   DBuf<uint8_t> tmask[kMaxDepth + 1];
   DBuf<int> act[kMaxDepth + 1], act_n[kMaxDepth + 1], act_scr;   // M2L target lists
   DBuf<uint8_t> smask;              // M2L skip_empty: source boxes of the level holding sources
-  DBuf<T> lapsr;                    // Laplace lane M2L: scaled operators of the level
+  DBuf<T> lapsr;                    // Laplace tile M2L: scaled operators of the level
   DBuf<T> hcx;                      // Helmholtz tile M2L: coaxial rows of the level
   DBuf<T> HE;                       // column M2L: rotation tables in even / odd blocks
-  DBuf<T> cols_cx;                  // and the level's coaxial tables
+  DBuf<T> cols_cx;                  // and the level's coaxial tables (lane M2L: its own)
+  DBuf<T> HL;                       // lane M2L: rotation tables
   DBuf<unsigned char> cols_tasks;   // and warp tiles
   DBuf<int> flag;
   // outputs (original order)
@@ -323,7 +324,7 @@ struct Solver : public wbfmm_b200_solver {
     f(n32_q); f(n32_dip); f(n32_nx); f(n32_ny); f(n32_nz); f(n32_pot); f(n32_grad);
     f(H64); f(H); f(op_ith); f(op_dist); f(op_r); f(op_ph); f(op_ch);
     for (int i = 0; i < 3; i++) { f(lap64[i]); f(lap[i]); }
-    f(partial); f(lin); f(lanes_part); f(act_scr); f(lapsr); f(hcx); f(HE); f(cols_cx); f(cols_tasks); f(smask); f(tc_part);
+    f(partial); f(lin); f(lanes_part); f(act_scr); f(lapsr); f(hcx); f(HE); f(HL); f(cols_cx); f(cols_tasks); f(smask); f(tc_part);
   }
 
   ~Solver() override {
@@ -722,7 +723,11 @@ struct Solver : public wbfmm_b200_solver {
     WBFMM_TRY(build_cols_rotations<T>(H64.p, hstride, nth, L, HE.p, stream));
     tables.HE = HE.p;
     tables.hestride = cols_rotation_stride<T>(L);
-    launches += 3;
+    WBFMM_TRY(HL.alloc((size_t)lane_rotation_stride<T>(L) * nth));
+    WBFMM_TRY(build_lane_rotations<T>(H64.p, hstride, nth, L, HL.p, stream));
+    tables.HL = HL.p;
+    tables.hlstride = lane_rotation_stride<T>(L);
+    launches += 4;
     if (helm) {
       WBFMM_TRY(helm_coaxial_set());
     } else {
@@ -909,6 +914,7 @@ struct Solver : public wbfmm_b200_solver {
       use_tiles = !use_lanes && tiles_ok;
     } else if (m2l_mode == 2) {
       use_lanes = lanes_ok;
+      use_tiles = !use_lanes && cols_ok;
     } else if (m2l_mode == 3) {
       use_tiles = tiles_ok;
     }
@@ -966,7 +972,7 @@ struct Solver : public wbfmm_b200_solver {
       // (box-major for target lists)
       const bool boxmajor = x.tmask && act[level].p;
       WBFMM_TRY(lin.alloc(lanes_lin_bytes(level, x.Nin, helm, sizeof(T))));
-      WBFMM_TRY((helm ? lanes_to_lin<T, true>(x.cin, level, x.Nin, 0, lin.p, stream, boxmajor)
+      WBFMM_TRY((helm ? cols_planes<T, true>(x.cin, level, x.Nin, 0, -1, lin.p, stream, boxmajor)
                       : lanes_to_lin<T, false>(x.cin, level, x.Nin, x.lap_e, lin.p, stream,
                                                boxmajor)));
       LanesParams<T> lp;
@@ -983,13 +989,7 @@ struct Solver : public wbfmm_b200_solver {
         lp.smask = smask.p;
         launches++;
       }
-      if (!helm) {
-        const int P1 = x.Nin + 1;
-        WBFMM_TRY(lapsr.alloc((size_t)kNumOps * P1 * P1 * P1));
-        WBFMM_TRY(build_lap_sr_ops<T>(tables, x.Nin, x.width, x.lap_e, lapsr.p, stream));
-        lp.lapsr = lapsr.p;
-        launches++;
-      }
+      WBFMM_TRY(lane_tables(lp));
       const int64_t np = (int64_t)1 << (3 * (level - 1));
       const int64_t base = ((np + 127) / 128) * 8;
       int ns = 1;
@@ -1017,6 +1017,16 @@ struct Solver : public wbfmm_b200_solver {
     launches += nsplit > 1 ? 2 : 1;
     return helm ? launch_m2l<T, true>(x, tables, stream)
                 : launch_m2l<T, false>(x, tables, stream);
+  }
+
+  // the level's coaxial tables of the lane kernel
+  int lane_tables(LanesParams<T>& lp) {
+    WBFMM_TRY(cols_cx.alloc(helm ? lane_coax_count<T, true>(lp.N) : lane_coax_count<T, false>(lp.N)));
+    WBFMM_TRY((helm ? build_lane_coax<T, true>(lp, tables, cols_cx.p, stream)
+                    : build_lane_coax<T, false>(lp, tables, cols_cx.p, stream)));
+    lp.lanes_cx = cols_cx.p;
+    launches++;
+    return 0;
   }
 
   // The M2L of a level as matrix products on columns of target boxes
@@ -1084,7 +1094,9 @@ struct Solver : public wbfmm_b200_solver {
     const int64_t G = ngroups[level];
     const int se = helm ? he : x.lap_e;
     WBFMM_TRY(lin.alloc(lanes_lin_groups_bytes(G, x.Nin, helm, sizeof(T))));
-    WBFMM_TRY((helm ? lanes_to_lin_groups<T, true>(x.cin, G, x.Nin, se, lin.p, stream, use_lanes)
+    WBFMM_TRY((helm ? use_lanes
+                          ? cols_planes<T, true>(x.cin, level, x.Nin, 0, G, lin.p, stream, true)
+                          : lanes_to_lin_groups<T, true>(x.cin, G, x.Nin, se, lin.p, stream, false)
                     : lanes_to_lin_groups<T, false>(x.cin, G, x.Nin, se, lin.p, stream, use_lanes)));
     WBFMM_TRY(pmap.alloc(source_mask_bytes(level) / 8));
     WBFMM_TRY(build_parent_slot_map(gmap[level].p, level, (uint32_t)G, pmap.p, stream));
@@ -1101,7 +1113,9 @@ struct Solver : public wbfmm_b200_solver {
     WBFMM_TRY(smask.alloc(source_mask_bytes(level)));
     WBFMM_TRY(build_source_mask(x.src_n, level, smask.p, stream));
     lp.smask = smask.p;
-    if (!helm) {
+    if (use_lanes) {
+      WBFMM_TRY(lane_tables(lp));
+    } else if (!helm) {
       const int P1 = x.Nin + 1;
       WBFMM_TRY(lapsr.alloc((size_t)kNumOps * P1 * P1 * P1));
       WBFMM_TRY(build_lap_sr_ops<T>(tables, x.Nin, x.width, x.lap_e, lapsr.p, stream));

@@ -70,6 +70,7 @@ struct TableCache {
     int nth = 0;
     double* H64 = nullptr; float* H32 = nullptr;
     double* HE64 = nullptr; float* HE32 = nullptr;
+    double* HL64 = nullptr; float* HL32 = nullptr;
     int* op_ith = nullptr; int* op_dist = nullptr;
     double* r64 = nullptr; float* r32 = nullptr;
     double* ph64 = nullptr; float* ph32 = nullptr;
@@ -91,7 +92,7 @@ struct TableCache {
   // release every table (no solve may be using them)
   void clear() {
     for (Geo* g : geos) {
-      void* ps[] = {g->H64, g->H32, g->HE64, g->HE32, g->op_ith, g->op_dist, g->r64, g->r32,
+      void* ps[] = {g->H64, g->H32, g->HE64, g->HE32, g->HL64, g->HL32, g->op_ith, g->op_dist, g->r64, g->r32,
                     g->ph64, g->ph32, g->ch64, g->ch32, g->lap64[0], g->lap64[1],
                     g->lap64[2], g->lap32[0], g->lap32[1], g->lap32[2]};
       for (void* p : ps) cudaFree(p);
@@ -131,7 +132,7 @@ struct TableCache {
   // release a Geo's tables and event (stream-ordered on s for pool memory)
   // and the Geo
   void drop_geo(Geo* g, cudaStream_t s) {
-    void* ps[] = {g->H64, g->H32, g->HE64, g->HE32, g->op_ith, g->op_dist, g->r64, g->r32,
+    void* ps[] = {g->H64, g->H32, g->HE64, g->HE32, g->HL64, g->HL32, g->op_ith, g->op_dist, g->r64, g->r32,
                   g->ph64, g->ph32, g->ch64, g->ch32, g->lap64[0], g->lap64[1],
                   g->lap64[2], g->lap32[0], g->lap32[1], g->lap32[2]};
     for (void* p : ps)
@@ -194,6 +195,10 @@ struct TableCache {
     WBFMM_CACHE_TRY(dalloc(g, &g->HE32, (size_t)cols_rotation_stride<float>(L) * g->nth, s));
     WBFMM_CACHE_TRY(build_cols_rotations(g->H64, g->hstride, g->nth, L, g->HE64, s));
     WBFMM_CACHE_TRY(build_cols_rotations(g->H64, g->hstride, g->nth, L, g->HE32, s));
+    WBFMM_CACHE_TRY(dalloc(g, &g->HL64, (size_t)lane_rotation_stride<double>(L) * g->nth, s));
+    WBFMM_CACHE_TRY(dalloc(g, &g->HL32, (size_t)lane_rotation_stride<float>(L) * g->nth, s));
+    WBFMM_CACHE_TRY(build_lane_rotations(g->H64, g->hstride, g->nth, L, g->HL64, s));
+    WBFMM_CACHE_TRY(build_lane_rotations(g->H64, g->hstride, g->nth, L, g->HL32, s));
     const size_t n3 = (size_t)(L + 1) * (L + 1) * (L + 1);
     for (int i = 0; i < 3; i++) {
       WBFMM_CACHE_TRY(dalloc(g, &g->lap64[i], n3, s));
@@ -228,6 +233,8 @@ struct TableCache {
     t->hstride = g->hstride;
     t->HE = f32 ? (const T*)g->HE32 : (const T*)g->HE64;
     t->hestride = cols_rotation_stride<T>(g->L);
+    t->HL = f32 ? (const T*)g->HL32 : (const T*)g->HL64;
+    t->hlstride = lane_rotation_stride<T>(g->L);
     t->op_ith = g->op_ith;
     t->op_dist = g->op_dist;
     t->op_r = f32 ? (const T*)g->r32 : (const T*)g->r64;
