@@ -62,23 +62,20 @@ int ensure_smem(size_t bytes) {
 // *a = va and, when b is non-null, *b = vb (one thread, on stream s)
 void launch_set_words(uint32_t* a, uint32_t va, uint32_t* b, uint32_t vb,
                       cudaStream_t s);
-// keys[i] = Morton key of point i (src/boxes.c:324-339); vals[i] = i.
+// keys[i] = Morton key of point i (src/boxes.c:324-339); vals[i] = i; with
+// bad non-null the strict-interior domain check of the sources
+// (src/boxes.c:148-153): *bad = min(*bad, first point outside).
 // f32: in FP32 arithmetic, as the single-precision build (the *_f API), on
 // coordinates, origin and width that are FP32 values
 void launch_point_keys(const double* pts, int64_t pstr, int n,
                        const double* x0, double D, uint64_t* keys,
-                       uint32_t* vals, cudaStream_t s, bool f32 = false);
+                       uint32_t* vals, int* bad, cudaStream_t s, bool f32 = false);
 // target leaf boxes by floor((x-x0)/wb) (src/boxes.c:585-634); vals[i] = i;
 // points outside the closed cube set *bad (host-visible flag) to 1
 void launch_target_keys(const double* pts, int64_t pstr, int n,
                         const double* x0, double D, int level,
                         uint64_t* keys, uint32_t* vals, int* bad,
                         cudaStream_t s, bool f32 = false);
-// strict-interior domain check of sources (src/boxes.c:148-153)
-void launch_domain_check(const double* pts, int64_t pstr, int n,
-                         const double* x0, double D, int* bad, cudaStream_t s,
-                         bool f32 = false);
-
 struct RadixScratch {
   uint64_t* keys_alt = nullptr;
   uint32_t* vals_alt = nullptr;
@@ -94,20 +91,24 @@ void radix_scratch_free(RadixScratch* scr);
 // curl[3 nt] from the gradients g[3][3 nt] of the three potential components
 int launch_curl_combine(const double* g, int nt, double* curl, cudaStream_t s);
 
-// box {i, n} of one level from the sorted keys, reproducing
-// wbfmm_tree_refine (src/boxes.c:208-277); parent_i is read before the
-// parents' .i advance, which launch_refine_parents then applies.
-void launch_refine_children(const uint64_t* sorted_keys, int npts,
-                            int level, const uint32_t* parent_i,
-                            uint32_t* child_i, uint32_t* child_n,
-                            cudaStream_t s);
-void launch_refine_parents(int level, uint32_t* parent_i,
-                           const uint32_t* parent_n, cudaStream_t s);
+// box {i, n} of levels 0..depth from the sorted keys, as `depth` calls of
+// wbfmm_tree_refine leave them (src/boxes.c:208-277)
+struct LevelBoxes {
+  uint32_t* i[kMaxDepth + 1];
+  uint32_t* n[kMaxDepth + 1];
+};
+void launch_refine_levels(const uint64_t* sorted_keys, int npts, int depth, const LevelBoxes& b,
+                          cudaStream_t s);
 // per-box start / count of sorted box ids (plain lower bounds; used for
 // the target bins)
 void launch_box_ranges(const uint64_t* sorted_ids, int n, int level,
                        uint32_t* start, uint32_t* count, cudaStream_t s);
 
+// targets = sources: perm = ip, positions, leaf boxes keys >> shift
+void launch_source_targets(const uint32_t* ip, const double* x, const double* y, const double* z,
+                           const uint64_t* keys, int shift, int n, uint32_t* perm, double* tx,
+                           double* ty, double* tz, uint64_t* tkeys, uint32_t* tbox,
+                           cudaStream_t s);
 // gathers into sorted order
 void launch_gather_points(const double* pts, int64_t pstr, const uint32_t* ip,
                           int n, double* x, double* y, double* z,

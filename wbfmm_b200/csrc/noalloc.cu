@@ -29,7 +29,7 @@ constexpr int kNoAllocTiles = (kNoAllocMaxPoints + 2047) / 2048;
 constexpr size_t kNaKeysOff = 0;
 constexpr size_t kNaValsOff = kNaKeysOff + sizeof(uint64_t) * (size_t)kNoAllocMaxPoints;
 constexpr size_t kNaHistOff = kNaValsOff + sizeof(uint32_t) * (size_t)kNoAllocMaxPoints;
-constexpr size_t kNaFlagOff = kNaHistOff + sizeof(uint32_t) * 256 * (size_t)kNoAllocTiles;
+constexpr size_t kNaFlagOff = kNaHistOff + sizeof(uint32_t) * 256 * (size_t)(kNoAllocTiles + 1);
 constexpr size_t kNaBytes = kNaFlagOff + 256;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNaBytes];
@@ -79,14 +79,13 @@ extern "C" int wbfmm_b200_morton_sort_noalloc(int n, const double* pts,
   // strict-interior domain check (src/boxes.c:148-153): the flag keeps the
   // last call's value, so a kernel on the caller's stream resets it first
   launch_set_words((uint32_t*)flag, 0x7fffffffu, nullptr, 0, s);
-  launch_domain_check(pts, pstr, n, x0, D, flag, s);
-  launch_point_keys(pts, pstr, n, x0, D, keys, ip, s);
+  launch_point_keys(pts, pstr, n, x0, D, keys, ip, flag, s);
   RadixScratch scr;
   scr.keys_alt = (uint64_t*)(base + kNaKeysOff);
   scr.vals_alt = (uint32_t*)(base + kNaValsOff);
   scr.hist = (uint32_t*)(base + kNaHistOff);
   scr.cap = (size_t)kNoAllocMaxPoints;
-  scr.hist_cap = (size_t)256 * kNoAllocTiles;
+  scr.hist_cap = (size_t)256 * (kNoAllocTiles + 1);
   // with cap and hist_cap covering n, radix_sort_pairs allocates nothing;
   // the histograms are fully rewritten by every pass
   rc = radix_sort_pairs(keys, ip, n, 60, &scr, s);

@@ -116,27 +116,11 @@ static __global__ void k_u64_to_u32(const uint64_t* __restrict__ a,
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) b[i] = (uint32_t)a[i];
 }
-// targets that are the sources: leaf box of each sorted source key
-static __global__ void k_leaf_of_keys(const uint64_t* __restrict__ keys, int shift,
-                                      uint64_t* __restrict__ tkeys,
-                                      uint32_t* __restrict__ tbox, int n) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint64_t b = keys[i] >> shift;
-  tkeys[i] = b;
-  tbox[i] = (uint32_t)b;
-}
-// box at `level` has targets below it
-static __global__ void k_target_mask(const uint32_t* __restrict__ leaf_count,
-                              int depth, int level, uint8_t* __restrict__ mask) {
-  int64_t nb = (int64_t)1 << (3 * level);
-  int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nb) return;
-  int sh = 3 * (depth - level);
-  int64_t lo = b << sh, hi = (b + 1) << sh;
-  uint8_t any = 0;
-  for (int64_t c = lo; c < hi && !any; c++) any = leaf_count[c] != 0;
-  mask[b] = any;
+// mask[b] = leaf box b holds targets
+static __global__ void k_target_mask(const uint32_t* __restrict__ leaf_count, int64_t n,
+                                     uint8_t* __restrict__ mask) {
+  const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (b < n) mask[b] = leaf_count[b] != 0;
 }
 
 // parent[b] = any of child[8 b .. 8 b + 7] (a target mask one level up)
@@ -455,21 +439,21 @@ struct Solver : public wbfmm_b200_solver {
     }
     // strict-interior domain check (src/boxes.c:148-153)
     launch_set_words((uint32_t*)flag.p, 0x7fffffffu, (uint32_t*)flag.p + 2, 0, stream);
-    launch_domain_check(dpts, xs_str, n, cfg.x0, cfg.D, flag.p, stream, cfg.keys_fp32 != 0);
+    WBFMM_TRY(keys.alloc(n));
+    WBFMM_TRY(ip.alloc(n));
+    launch_point_keys(dpts, xs_str, n, cfg.x0, cfg.D, keys.p, ip.p, flag.p, stream,
+                      cfg.keys_fp32 != 0);
     if (!async_checks) {
       int bad = 0;
       WBFMM_CUDA(cudaMemcpyAsync(&bad, flag.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
       WBFMM_CUDA(cudaStreamSynchronize(stream));
       WBFMM_TRY(domain_error(bad, 0));
     }
-    WBFMM_TRY(keys.alloc(n));
-    WBFMM_TRY(ip.alloc(n));
-    launch_point_keys(dpts, xs_str, n, cfg.x0, cfg.D, keys.p, ip.p, stream, cfg.keys_fp32 != 0);
     // full 60-bit keys (the reference's point order), or with leaf_order
     // only the bits that select the leaf box
     const int sort_lo = cfg.leaf_order ? 60 - 3 * depth : 0;
     WBFMM_TRY(radix_sort_pairs(keys.p, ip.p, n, 60 - sort_lo, &rs, stream, sort_lo));
-    launches += 4 + 3 * ((60 - sort_lo + 7) / 8);
+    launches += 2 + (n <= 4096 ? 1 : 3 * ((60 - sort_lo + 7) / 8));
     WBFMM_TRY(sx.alloc(n)); WBFMM_TRY(sy.alloc(n)); WBFMM_TRY(sz.alloc(n));
     launch_gather_points(dpts, xs_str, ip.p, n, sx.p, sy.p, sz.p, stream);
     launches++;
@@ -493,15 +477,15 @@ struct Solver : public wbfmm_b200_solver {
       launches += 4;
     }
     // levels: box {i, n} by repeated refinement (src/boxes.c:208-277)
-    WBFMM_TRY(box_i[0].alloc(1)); WBFMM_TRY(box_n[0].alloc(1));
-    launch_set_words(box_i[0].p, 0u, box_n[0].p, (uint32_t)n, stream);
-    for (int l = 1; l <= depth; l++) {
+    LevelBoxes lb;
+    for (int l = 0; l <= depth; l++) {
       size_t nb = (size_t)1 << (3 * l);
       WBFMM_TRY(box_i[l].alloc(nb)); WBFMM_TRY(box_n[l].alloc(nb));
-      launch_refine_children(keys.p, n, l, box_i[l - 1].p, box_i[l].p, box_n[l].p, stream);
-      launch_refine_parents(l - 1, box_i[l - 1].p, box_n[l - 1].p, stream);
-      launches += 2;
+      lb.i[l] = box_i[l].p;
+      lb.n[l] = box_n[l].p;
     }
+    launch_refine_levels(keys.p, n, depth, lb, stream);
+    launches++;
     WBFMM_CUDA(cudaGetLastError());
     // coefficient arrays (arrays adopted from the caller are kept; sparse
     // storage allocates once the targets are known, prepare_sparse)
@@ -561,12 +545,8 @@ struct Solver : public wbfmm_b200_solver {
       // the sources' array again: the source sort already groups the points
       // by leaf box (the order inside a leaf changes no target's field), and
       // the sources passed the domain check
-      WBFMM_CUDA(cudaMemcpyAsync(tperm.p, ip.p, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, stream));
-      WBFMM_CUDA(cudaMemcpyAsync(tx.p, sx.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, stream));
-      WBFMM_CUDA(cudaMemcpyAsync(ty.p, sy.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, stream));
-      WBFMM_CUDA(cudaMemcpyAsync(tz.p, sz.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, stream));
-      k_leaf_of_keys<<<(n + 255) / 256, 256, 0, stream>>>(keys.p, 60 - 3 * depth, tkeys.p,
-                                                         tbox.p, n);
+      launch_source_targets(ip.p, sx.p, sy.p, sz.p, keys.p, 60 - 3 * depth, n, tperm.p, tx.p, ty.p,
+                            tz.p, tkeys.p, tbox.p, stream);
       launches++;
     } else {
       const double* d = xt;
@@ -581,18 +561,20 @@ struct Solver : public wbfmm_b200_solver {
       WBFMM_TRY(radix_sort_pairs(tkeys.p, tperm.p, n, 3 * depth, &rs, stream));
       launch_gather_points(d, tstr, tperm.p, n, tx.p, ty.p, tz.p, stream);
       k_u64_to_u32<<<(n + 255) / 256, 256, 0, stream>>>(tkeys.p, tbox.p, n);
-      launches += 3 + 3 * ((3 * depth + 7) / 8);
+      launches += 3 + (n <= 4096 ? 1 : 3 * ((3 * depth + 7) / 8));
     }
     size_t nb = (size_t)1 << (3 * depth);
     WBFMM_TRY(tstart.alloc(nb)); WBFMM_TRY(tcount.alloc(nb));
     launch_box_ranges(tkeys.p, n, depth, tstart.p, tcount.p, stream);
     launches++;
     if (cfg.skip_empty) {
-      for (int l = 2; l <= depth; l++) {
-        size_t nbl = (size_t)1 << (3 * l);
-        WBFMM_TRY(tmask[l].alloc(nbl));
-        k_target_mask<<<(unsigned)((nbl + 255) / 256), 256, 0, stream>>>(
-            tcount.p, depth, l, tmask[l].p);
+      // leaf masks from the counts, each level above from the one below
+      for (int l = depth; l >= 2; l--) {
+        const int64_t nbl = (int64_t)1 << (3 * l);
+        WBFMM_TRY(tmask[l].alloc((size_t)nbl));
+        const unsigned g = (unsigned)((nbl + 255) / 256);
+        if (l == depth) k_target_mask<<<g, 256, 0, stream>>>(tcount.p, nbl, tmask[l].p);
+        else k_mask_up<<<g, 256, 0, stream>>>(tmask[l + 1].p, nbl, tmask[l].p);
         // the M2L kernels' per-child-type lists of the boxes with targets
         WBFMM_TRY(act[l].alloc(nbl));
         WBFMM_TRY(act_n[l].alloc(8));

@@ -36,34 +36,6 @@ __device__ __forceinline__ uint32_t key_coord(double x, double x0, double D, boo
   return (uint32_t)(__ddiv_rn(__dsub_rn(x, x0), D) * 1048576.0);
 }
 
-__global__ void k_point_keys(const double* __restrict__ pts, int64_t pstr,
-                             int n, double x0, double y0, double z0, double D,
-                             uint64_t* __restrict__ keys,
-                             uint32_t* __restrict__ vals, bool f32) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double* p = pts + (int64_t)i * pstr;
-  uint32_t xi = key_coord(p[0], x0, D, f32);
-  uint32_t yi = key_coord(p[1], y0, D, f32);
-  uint32_t zi = key_coord(p[2], z0, D, f32);
-  // Points strictly inside the cube give 20-bit coordinates.  Anything else
-  // (rejected by the domain check, which the served form reads back only
-  // after the solve) is clamped so every key stays below 2^60 and every box
-  // index derived from it inside its level's array.
-  const uint32_t top = (1u << 20) - 1;
-  xi = xi < top ? xi : top; yi = yi < top ? yi : top; zi = zi < top ? zi : top;
-  keys[i] = morton(xi, yi, zi);
-  vals[i] = (uint32_t)i;
-}
-
-void launch_point_keys(const double* pts, int64_t pstr, int n,
-                       const double* x0, double D, uint64_t* keys,
-                       uint32_t* vals, cudaStream_t s, bool f32) {
-  if (n <= 0) return;
-  k_point_keys<<<(n + 255) / 256, 256, 0, s>>>(pts, pstr, n, x0[0], x0[1],
-                                               x0[2], D, keys, vals, f32);
-}
-
 // wbfmm_point_box (src/boxes.c:585-634); with f32 in FP32 arithmetic
 __device__ __forceinline__ bool outside_closed(double x, double x0, double D, bool f32) {
   if (f32) {
@@ -139,30 +111,47 @@ __device__ __forceinline__ bool outside_open(double x, double x0, double D, bool
   return x <= x0 || x >= x0 + D;
 }
 
-__global__ void k_domain_check(const double* __restrict__ pts, int64_t pstr,
-                               int n, double x0, double y0, double z0,
-                               double D, int* bad, bool f32) {
+// the key of every point, and with `bad` the strict-interior check: *bad the
+// first point outside
+__global__ void k_point_keys(const double* __restrict__ pts, int64_t pstr,
+                             int n, double x0, double y0, double z0, double D,
+                             uint64_t* __restrict__ keys,
+                             uint32_t* __restrict__ vals, int* bad, bool f32) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double* p = pts + (int64_t)i * pstr;
-  if (outside_open(p[0], x0, D, f32) || outside_open(p[1], y0, D, f32) ||
-      outside_open(p[2], z0, D, f32))
+  const double x = p[0], y = p[1], z = p[2];
+  if (bad && (outside_open(x, x0, D, f32) || outside_open(y, y0, D, f32) ||
+              outside_open(z, z0, D, f32)))
     atomicMin(bad, i);
+  uint32_t xi = key_coord(x, x0, D, f32);
+  uint32_t yi = key_coord(y, y0, D, f32);
+  uint32_t zi = key_coord(z, z0, D, f32);
+  // Points strictly inside the cube give 20-bit coordinates.  Anything else
+  // (rejected by the domain check, which the served form reads back only
+  // after the solve) is clamped so every key stays below 2^60 and every box
+  // index derived from it inside its level's array.
+  const uint32_t top = (1u << 20) - 1;
+  xi = xi < top ? xi : top; yi = yi < top ? yi : top; zi = zi < top ? zi : top;
+  keys[i] = morton(xi, yi, zi);
+  vals[i] = (uint32_t)i;
 }
 
-void launch_domain_check(const double* pts, int64_t pstr, int n,
-                         const double* x0, double D, int* bad, cudaStream_t s,
-                         bool f32) {
+void launch_point_keys(const double* pts, int64_t pstr, int n,
+                       const double* x0, double D, uint64_t* keys,
+                       uint32_t* vals, int* bad, cudaStream_t s, bool f32) {
   if (n <= 0) return;
-  k_domain_check<<<(n + 255) / 256, 256, 0, s>>>(pts, pstr, n, x0[0], x0[1],
-                                                 x0[2], D, bad, f32);
+  k_point_keys<<<(n + 255) / 256, 256, 0, s>>>(pts, pstr, n, x0[0], x0[1],
+                                               x0[2], D, keys, vals, bad, f32);
 }
 
 // ------------------------------------------------------------ radix sort
 // Stable LSD radix sort, 8-bit digits.  Each pass: per-tile digit
-// histograms (digit-major), one exclusive scan, then a scatter in which
-// every tile ranks its elements round by round (warp match + per-warp
-// digit counts), which keeps equal digits in input order.
+// histograms (digit-major), an exclusive scan of every digit's row (a CTA
+// per digit) with the digits' totals, then a scatter in which every tile
+// scans the totals, ranks its elements round by round (warp match + per-warp
+// digit counts), which keeps equal digits in input order.  Up to
+// kSmallSort elements, one CTA runs every pass in shared memory.
 constexpr int kSortThreads = 256;
 constexpr int kSortItems = 8;
 constexpr int kSortTile = kSortThreads * kSortItems;
@@ -181,40 +170,58 @@ __global__ void k_radix_hist(const uint64_t* __restrict__ keys, int n, int shift
   hist[threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
 }
 
-// exclusive scan of m entries by one block of 1024 threads
-__global__ void k_scan_exclusive(uint32_t* data, int m) {
-  __shared__ uint32_t sums[1024];
-  int t = threadIdx.x;
-  int per = (m + 1023) / 1024;
-  int lo = t * per, hi = min(lo + per, m);
-  uint32_t s = 0;
-  for (int i = lo; i < hi; i++) s += data[i];
-  sums[t] = s;
+// exclusive sum over the 256 threads of a CTA (s_w: 8 words), *total the sum
+__device__ __forceinline__ uint32_t scan256(uint32_t v, uint32_t* s_w, uint32_t* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t x = v;
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t u = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += u;
+  }
+  if (lane == 31) s_w[warp] = x;
   __syncthreads();
-  for (int off = 1; off < 1024; off <<= 1) {
-    uint32_t v = t >= off ? sums[t - off] : 0;
-    __syncthreads();
-    sums[t] += v;
-    __syncthreads();
+  uint32_t before = 0, all = 0;
+  for (int w = 0; w < 8; w++) {
+    if (w < warp) before += s_w[w];
+    all += s_w[w];
   }
-  uint32_t run = t > 0 ? sums[t - 1] : 0;
-  for (int i = lo; i < hi; i++) {
-    uint32_t v = data[i];
-    data[i] = run;
-    run += v;
+  __syncthreads();
+  *total = all;
+  return before + x - v;
+}
+
+// a digit's row of tile counts -> exclusive sums, its total to totals[digit].
+// The tiles of a million points are 489 per digit: one CTA scanning all 125
+// thousand counts took 0.10 ms a pass, a third of an 8-pass sort of 2e6 points
+__global__ void k_scan_rows(uint32_t* __restrict__ hist, int ntiles,
+                            uint32_t* __restrict__ totals) {
+  __shared__ uint32_t s_w[8];
+  uint32_t* row = hist + (size_t)blockIdx.x * ntiles;
+  uint32_t carry = 0;
+  for (int b = 0; b < ntiles; b += 256) {
+    const int i = b + threadIdx.x;
+    const uint32_t v = i < ntiles ? row[i] : 0;
+    uint32_t all;
+    const uint32_t ex = scan256(v, s_w, &all);
+    if (i < ntiles) row[i] = carry + ex;
+    carry += all;
   }
+  if (threadIdx.x == 0) totals[blockIdx.x] = carry;
 }
 
 __global__ void k_radix_scatter(const uint64_t* __restrict__ keys,
                                 const uint32_t* __restrict__ vals, int n,
                                 int shift, int ntiles,
                                 const uint32_t* __restrict__ offs,
+                                const uint32_t* __restrict__ totals,
                                 uint64_t* __restrict__ okeys,
                                 uint32_t* __restrict__ ovals) {
   __shared__ uint32_t base[256];
   __shared__ uint32_t wcnt[kSortThreads / 32][256];
+  __shared__ uint32_t s_w[8];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  base[t] = offs[t * ntiles + blockIdx.x];
+  uint32_t all;
+  base[t] = scan256(totals[t], s_w, &all) + offs[t * ntiles + blockIdx.x];
   int tile0 = blockIdx.x * kSortTile;
   for (int r = 0; r < kSortItems; r++) {
     for (int w = 0; w < kSortThreads / 32; w++) wcnt[w][t] = 0;
@@ -246,6 +253,74 @@ __global__ void k_radix_scatter(const uint64_t* __restrict__ keys,
   }
 }
 
+// The whole sort of n <= kSmallSort pairs by one CTA: every pass in shared
+// memory (1000 points, 8 passes: 24 launches, 0.13 ms, as separate kernels)
+constexpr int kSmallSort = 4096;
+constexpr size_t kSmallSortBytes =
+    2 * kSmallSort * (sizeof(uint64_t) + sizeof(uint32_t)) + (32 + 1) * 256 * sizeof(uint32_t);
+__global__ void __launch_bounds__(1024, 1)
+k_radix_small(uint64_t* __restrict__ keys, uint32_t* __restrict__ vals, int n, int lo, int passes) {
+  extern __shared__ __align__(16) unsigned char sort_sm[];
+  uint64_t* ka = (uint64_t*)sort_sm;
+  uint64_t* kb = ka + kSmallSort;
+  uint32_t* va = (uint32_t*)(kb + kSmallSort);
+  uint32_t* vb = va + kSmallSort;
+  uint32_t* wcnt = vb + kSmallSort;       // [32][256]
+  uint32_t* base = wcnt + 32 * 256;
+  __shared__ uint32_t s_w[8];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  for (int i = t; i < n; i += 1024) { ka[i] = keys[i]; va[i] = vals[i]; }
+  for (int p = 0; p < passes; p++) {
+    const int shift = lo + 8 * p;
+    if (t < 256) base[t] = 0;
+    __syncthreads();
+    for (int i = t; i < n; i += 1024) atomicAdd(&base[(ka[i] >> shift) & 0xff], 1u);
+    __syncthreads();
+    // first place of every digit: warps 0-7 scan, the others keep the barriers
+    uint32_t v = t < 256 ? base[t] : 0, x = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += u;
+    }
+    if (t < 256 && lane == 31) s_w[warp] = x;
+    __syncthreads();
+    if (t < 256) {
+      for (int w = 0; w < warp; w++) x += s_w[w];
+      base[t] = x - v;
+    }
+    for (int r = 0; r < n; r += 1024) {
+      for (int i = t; i < 32 * 256; i += 1024) wcnt[i] = 0;
+      __syncthreads();
+      const int i = r + t;
+      const bool valid = i < n;
+      const uint64_t key = valid ? ka[i] : 0;
+      const uint32_t d = valid ? (uint32_t)((key >> shift) & 0xff) : 256u + lane;
+      const unsigned peers = __match_any_sync(0xffffffffu, d);
+      const int rank = __popc(peers & ((1u << lane) - 1));
+      if (valid && rank == 0) wcnt[warp * 256 + d] = __popc(peers);
+      __syncthreads();
+      if (t < 256) {
+        uint32_t c[32], run = base[t];
+#pragma unroll
+        for (int w = 0; w < 32; w++) c[w] = wcnt[w * 256 + t];
+#pragma unroll
+        for (int w = 0; w < 32; w++) { wcnt[w * 256 + t] = run; run += c[w]; }
+        base[t] = run;
+      }
+      __syncthreads();
+      if (valid) {
+        const uint32_t pos = wcnt[warp * 256 + d] + rank;
+        kb[pos] = key;
+        vb[pos] = va[i];
+      }
+      __syncthreads();
+    }
+    uint64_t* tk = ka; ka = kb; kb = tk;
+    uint32_t* tv = va; va = vb; vb = tv;
+  }
+  for (int i = t; i < n; i += 1024) { keys[i] = ka[i]; vals[i] = va[i]; }
+}
+
 cudaMemPool_t library_pool();   // solver.cu
 
 // Growth of the sort's scratch, stream-ordered from the library's pool: a
@@ -263,6 +338,13 @@ static cudaError_t scratch_regrow(X** p, size_t count, cudaStream_t s) {
 int radix_sort_pairs(uint64_t* keys, uint32_t* vals, int n, int bits,
                      RadixScratch* scr, cudaStream_t s, int lo) {
   if (n <= 1) return 0;
+  int passes = (bits + 7) / 8;
+  if (n <= kSmallSort) {
+    WBFMM_SMEM(kSmallSortBytes, k_radix_small);
+    k_radix_small<<<1, 1024, kSmallSortBytes, s>>>(keys, vals, n, lo, passes);
+    WBFMM_CUDA(cudaGetLastError());
+    return 0;
+  }
   int ntiles = (n + kSortTile - 1) / kSortTile;
   if (scr->cap < (size_t)n) {
     scr->cap = 0;
@@ -270,20 +352,20 @@ int radix_sort_pairs(uint64_t* keys, uint32_t* vals, int n, int bits,
     WBFMM_CUDA(scratch_regrow(&scr->vals_alt, (size_t)n, s));
     scr->cap = n;
   }
-  if (scr->hist_cap < (size_t)ntiles * 256) {
+  if (scr->hist_cap < (size_t)(ntiles + 1) * 256) {
     scr->hist_cap = 0;
-    WBFMM_CUDA(scratch_regrow(&scr->hist, (size_t)256 * ntiles, s));
-    scr->hist_cap = (size_t)ntiles * 256;
+    WBFMM_CUDA(scratch_regrow(&scr->hist, (size_t)256 * (ntiles + 1), s));
+    scr->hist_cap = (size_t)(ntiles + 1) * 256;
   }
-  int passes = (bits + 7) / 8;
+  uint32_t* totals = scr->hist + (size_t)256 * ntiles;
   uint64_t *ki = keys, *ko = scr->keys_alt;
   uint32_t *vi = vals, *vo = scr->vals_alt;
   for (int p = 0; p < passes; p++) {
     int shift = lo + 8 * p;
     k_radix_hist<<<ntiles, kSortThreads, 0, s>>>(ki, n, shift, ntiles, scr->hist);
-    k_scan_exclusive<<<1, 1024, 0, s>>>(scr->hist, 256 * ntiles);
+    k_scan_rows<<<256, 256, 0, s>>>(scr->hist, ntiles, totals);
     k_radix_scatter<<<ntiles, kSortThreads, 0, s>>>(ki, vi, n, shift, ntiles,
-                                                    scr->hist, ko, vo);
+                                                    scr->hist, totals, ko, vo);
     uint64_t* tk = ki; ki = ko; ko = tk;
     uint32_t* tv = vi; vi = vo; vo = tv;
   }
@@ -315,46 +397,43 @@ __device__ __forceinline__ uint32_t lower_bound_box(const uint64_t* keys,
   return lo;
 }
 
-// Child c of parent P (level `level` boxes):
+// The boxes of every level 0..depth as `depth` refinements leave them
+// (src/boxes.c:208-277), in one launch.  Refining parent P (level - 1) gives
+// child c
 //   n = number of points in c;
 //   i = P.i (before refinement) for the first child; for the others, the
 //       sorted position of c's first point when the reference's scan
-//       reaches c (i.e. c is not past the parent's last point), else 0.
-__global__ void k_refine_children(const uint64_t* __restrict__ keys, int npts,
-                                  int level, const uint32_t* __restrict__ pi,
-                                  uint32_t* __restrict__ ci,
-                                  uint32_t* __restrict__ cn) {
-  int64_t nb = (int64_t)1 << (3 * level);
-  int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nb) return;
-  int shift = 3 * (20 - level);
-  uint32_t lb = lower_bound_box(keys, npts, shift, (uint64_t)c);
-  uint32_t ub = lower_bound_box(keys, npts, shift, (uint64_t)c + 1);
-  uint32_t pend = lower_bound_box(keys, npts, shift, (uint64_t)((c | 7) + 1));
-  cn[c] = ub - lb;
-  if ((c & 7) == 0) ci[c] = pi[c >> 3];
-  else ci[c] = lb < pend ? lb : 0u;
+//       reaches c (i.e. c is not past the parent's last point), else 0;
+// and then advances P.i by P.n.  A box that is a first child over several
+// levels takes the i of the highest of those boxes, whose first position is
+// its own: `a`, the ancestor by the trailing zero digits (i = 0 from the root).
+__global__ void k_refine_levels(const uint64_t* __restrict__ keys, int npts, int depth,
+                                LevelBoxes b) {
+  int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  int l = 0;
+  while (l <= depth && e >= ((int64_t)1 << (3 * l))) { e -= (int64_t)1 << (3 * l); l++; }
+  if (l > depth) return;
+  const int shift = 3 * (20 - l);
+  const uint64_t c = (uint64_t)e;
+  const uint32_t lb = lower_bound_box(keys, npts, shift, c);
+  const uint32_t ub = lower_bound_box(keys, npts, shift, c + 1);
+  uint64_t a = c;
+  int la = l;
+  while (la > 0 && (a & 7) == 0) { a >>= 3; la--; }
+  uint32_t i = 0;
+  if (la > 0) {
+    const uint32_t pend = lower_bound_box(keys, npts, 3 * (20 - la), (a | 7) + 1);
+    i = lb < pend ? lb : 0u;
+  }
+  b.n[l][e] = ub - lb;
+  b.i[l][e] = l < depth ? i + (ub - lb) : i;
 }
 
-__global__ void k_refine_parents(int64_t np, uint32_t* __restrict__ pi,
-                                 const uint32_t* __restrict__ pn) {
-  int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < np) pi[p] += pn[p];
-}
-
-void launch_refine_children(const uint64_t* sorted_keys, int npts, int level,
-                            const uint32_t* parent_i, uint32_t* child_i,
-                            uint32_t* child_n, cudaStream_t s) {
-  int64_t nb = (int64_t)1 << (3 * level);
-  k_refine_children<<<(unsigned)((nb + 255) / 256), 256, 0, s>>>(
-      sorted_keys, npts, level, parent_i, child_i, child_n);
-}
-
-void launch_refine_parents(int level, uint32_t* parent_i,
-                           const uint32_t* parent_n, cudaStream_t s) {
-  int64_t np = (int64_t)1 << (3 * level);
-  k_refine_parents<<<(unsigned)((np + 255) / 256), 256, 0, s>>>(np, parent_i,
-                                                                parent_n);
+void launch_refine_levels(const uint64_t* sorted_keys, int npts, int depth, const LevelBoxes& b,
+                          cudaStream_t s) {
+  int64_t tot = 0;
+  for (int l = 0; l <= depth; l++) tot += (int64_t)1 << (3 * l);
+  k_refine_levels<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(sorted_keys, npts, depth, b);
 }
 
 __global__ void k_box_ranges(const uint64_t* __restrict__ ids, int n,
@@ -391,6 +470,31 @@ void launch_gather_points(const double* pts, int64_t pstr, const uint32_t* ip,
                           cudaStream_t s) {
   if (n <= 0) return;
   k_gather_points<<<(n + 255) / 256, 256, 0, s>>>(pts, pstr, ip, n, x, y, z);
+}
+
+// targets that are the sources: their order, positions and leaf boxes
+__global__ void k_source_targets(const uint32_t* __restrict__ ip, const double* __restrict__ x,
+                                 const double* __restrict__ y, const double* __restrict__ z,
+                                 const uint64_t* __restrict__ keys, int shift, int n,
+                                 uint32_t* __restrict__ perm, double* __restrict__ tx,
+                                 double* __restrict__ ty, double* __restrict__ tz,
+                                 uint64_t* __restrict__ tkeys, uint32_t* __restrict__ tbox) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  perm[i] = ip[i];
+  tx[i] = x[i]; ty[i] = y[i]; tz[i] = z[i];
+  const uint64_t b = keys[i] >> shift;
+  tkeys[i] = b;
+  tbox[i] = (uint32_t)b;
+}
+
+void launch_source_targets(const uint32_t* ip, const double* x, const double* y, const double* z,
+                           const uint64_t* keys, int shift, int n, uint32_t* perm, double* tx,
+                           double* ty, double* tz, uint64_t* tkeys, uint32_t* tbox,
+                           cudaStream_t s) {
+  if (n <= 0) return;
+  k_source_targets<<<(n + 255) / 256, 256, 0, s>>>(ip, x, y, z, keys, shift, n, perm, tx, ty, tz,
+                                                   tkeys, tbox);
 }
 
 template <typename T>
