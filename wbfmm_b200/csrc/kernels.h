@@ -83,14 +83,16 @@ struct XlateParams {
   int Nin, Nout;      // orders of input and output expansions
   const T* cin;       // input level array (Layout L)
   T* cout;            // output level array (Layout L)
-  const uint32_t* src_n;   // M2L: source box counts (skip empty), or null
+  const uint32_t* src_n;   // M2L: source box counts (skip empty), or null; M2M: the
+                           // parents' (those without sources get zeros), or null
   const T* coax;           // Helmholtz coaxial table(s) for this level
   int64_t coax_stride;     // per distance (complex S|R)
   T width;                 // box width of the translation's distance unit
   T k;
   int nsplit;              // M2L: CTAs per target box
   T* partial;              // M2L split: [nsplit][nbox][2*ncout]
-  const uint8_t* tmask;    // M2L: only targets with tmask[b] != 0, or null
+  const uint8_t* tmask;    // M2L: only targets with tmask[b] != 0, or null; L2L: the
+                           // parents' (children of the others get zeros), or null
   int lap_e;               // Laplace M2L scale exponent (lap_scale_exp)
   // sparse storage (M2M, L2L): one CTA per slot of the child level
   // (nbox = its slots), glist its slot -> group (the parent box), gmap the

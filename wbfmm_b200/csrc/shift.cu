@@ -285,6 +285,13 @@ __global__ void k_m2m(XlateParams<T> p, OpTables<T> t) {
   const int64_t Pout = p.glist ? compact_box(p.gmap, (int64_t)p.glist[P]) : P;
   if (Pout < 0) return;   // (a stored group's parent is stored) whole CTA, before any barrier
   const int outlen = vlen<HELM>(Np);
+  if (p.src_n && p.src_n[p.glist ? (int64_t)p.glist[P] : P] == 0) {
+    // no sources below: zeros (whole CTA, before any barrier)
+    for (int c = threadIdx.x; c < 2 * outlen; c += blockDim.x) ((T*)smraw)[c] = T(0);
+    __syncthreads();
+    store_vec<T, HELM, false>(p.cout, Pout, Np, ncoef(Np), (T*)smraw, threadIdx.x, blockDim.x);
+    return;
+  }
   for (int c = lane; c < 2 * outlen; c += 32) acc[c] = T(0);
   if (!HELM && threadIdx.x == 0) {
     T r = p.width * (T)t.op_r[kOpM2M];
@@ -346,6 +353,12 @@ __global__ void k_l2l(XlateParams<T> p, OpTables<T> t) {
   const int64_t P = blockIdx.x;
   const int64_t Pin = p.glist ? compact_box(p.gmap, (int64_t)p.glist[P]) : P;
   if (Pin < 0) return;    // (a stored group's parent is stored) whole CTA, before any barrier
+  if (p.tmask && !p.tmask[p.glist ? (int64_t)p.glist[P] : P]) {
+    // no targets below: zeros (whole CTA, before any barrier)
+    const int64_t len = (int64_t)8 * ncoef(Nc) * (HELM ? 2 : 1);
+    for (int64_t c = threadIdx.x; c < len; c += blockDim.x) p.cout[P * len + c] = T(0);
+    return;
+  }
   if (!HELM && threadIdx.x == 0) {
     T r = p.width * (T)t.op_r[kOpL2L];
     tp[0] = T(1);

@@ -826,6 +826,9 @@ struct Solver : public wbfmm_b200_solver {
     x.cin = mps[level].p; x.cout = mps[level - 1].p;
     x.coax = helm ? ss_ptr[level] : nullptr;
     x.width = (T)width(level);
+    // skip_empty: the leaf expansions of boxes without sources are zeros
+    // (unless P2M adds to what the arrays hold)
+    if (cfg.skip_empty && !p2m_accumulate) x.src_n = box_n[level - 1].p;
     if (cfg.sparse) {
       // one CTA per stored group of the children; the parents' other
       // siblings (no sources or targets) hold zeros
@@ -1191,6 +1194,7 @@ struct Solver : public wbfmm_b200_solver {
     d.cin = mpr[level].p; d.cout = mpr[level + 1].p;
     d.coax = helm ? ss_ptr[level + 1] : nullptr;
     d.width = (T)width(level + 1);
+    if (cfg.skip_empty && tmask[level].p) d.tmask = tmask[level].p;
     if (cfg.sparse) {
       // one CTA per stored group of the children (every box of a stored
       // group is written)

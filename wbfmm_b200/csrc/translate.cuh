@@ -26,15 +26,27 @@ HD float scale2(float x, int e) { return ldexpf(x, e); }
 HD double scale2(double x, int e) { return ldexp(x, e); }
 HD int nhalf(int p) { return (p + 1) * (p + 2) / 2; }
 
+// square root for the degrees below, which correct it: on the device the FP32
+// approximation alone (an FP64 square root is some 30 instructions, and the
+// translation kernels take one per coefficient and stage)
+HD int root_floor(float x) {
+#ifdef __CUDA_ARCH__
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return (int)r;
+#else
+  return (int)sqrtf(x);
+#endif
+}
 // degree of flattened full index c = n(n+1)+m
 HD int full_degree(int c) {
-  int n = (int)sqrt((double)c);
+  int n = root_floor((float)c);
   while ((n + 1) * (n + 1) <= c) n++;
   while (n * n > c) n--;
   return n;
 }
 HD int half_degree(int c) {
-  int n = (int)((sqrt(8.0 * c + 1.0) - 1.0) * 0.5);
+  int n = (root_floor(8.0f * c + 1.0f) - 1) / 2;
   while ((n + 1) * (n + 2) / 2 <= c) n++;
   while (n * (n + 1) / 2 > c) n--;
   return n;
