@@ -63,6 +63,45 @@ __device__ __forceinline__ void sincos_near(float x, float* sp, float* cp) {
   *cp = co;
 }
 
+// sin and cos of x >= 0 in FP64 for the near field, the same reduction (its
+// constants pi/2 and pi/2 - fl(pi/2) in FP64) and the Taylor series to r^17
+// and r^18 (truncation below 1e-19 at |r| = pi/4): about 40 instructions.  The
+// library's sincos serves arguments where the two-constant reduction would
+// lose digits.
+__device__ __forceinline__ void sincos_near(double x, double* sp, double* cp) {
+  if (x > 1e5) {
+    sincos(x, sp, cp);
+    return;
+  }
+  const double q = rint(x * 0.63661977236758134308);
+  double r = fma(-q, 1.57079632679489655800, x);
+  r = fma(-q, 6.12323399573676603587e-17, r);
+  const double r2 = r * r;
+  double ps = 1.0 / 355687428096000.0;                      // 1/17!
+  ps = fma(r2, ps, -1.0 / 1307674368000.0);
+  ps = fma(r2, ps, 1.0 / 6227020800.0);
+  ps = fma(r2, ps, -1.0 / 39916800.0);
+  ps = fma(r2, ps, 1.0 / 362880.0);
+  ps = fma(r2, ps, -1.0 / 5040.0);
+  ps = fma(r2, ps, 1.0 / 120.0);
+  ps = fma(r2, ps, -1.0 / 6.0);
+  const double sn = fma(r * r2, ps, r);
+  double pc = -1.0 / 6402373705728000.0;                    // 1/18!
+  pc = fma(r2, pc, 1.0 / 20922789888000.0);
+  pc = fma(r2, pc, -1.0 / 87178291200.0);
+  pc = fma(r2, pc, 1.0 / 479001600.0);
+  pc = fma(r2, pc, -1.0 / 3628800.0);
+  pc = fma(r2, pc, 1.0 / 40320.0);
+  pc = fma(r2, pc, -1.0 / 720.0);
+  pc = fma(r2, pc, 1.0 / 24.0);
+  pc = fma(r2, pc, -0.5);
+  const double cn = fma(r2, pc, 1.0);
+  const int n = (int)q;
+  const double so = (n & 1) ? cn : sn, co = (n & 1) ? sn : cn;
+  *sp = (n & 2) ? -so : so;
+  *cp = ((n + 1) & 2) ? -co : co;
+}
+
 // The terms of one (target, source) pair at separation r = (rx, ry, rz)
 // (|r|^2 = r2) added to acc[0..] (Helmholtz: pot re, im, then grad x re,
 // x im, y, z; Laplace: pot, grad x, y, z), without the kernels' constant
@@ -89,14 +128,9 @@ __device__ __forceinline__ void p2p_pair(const P2PTile<T, HELM, NT>& tl, int j, 
   const T ir = MASKED ? (r2 > rc2 ? pair_rsqrt(r2) : T(0)) : pair_rsqrt(r2);
   if (HELM) {
     const T r = r2 * ir;
-    T kr = k * r, ikr, sn, cs;
-    if constexpr (sizeof(T) == 4) {
-      ikr = ir * kinv;
-      sincos_near(kr, &sn, &cs);
-    } else {
-      ikr = ir / k;
-      sincos(kr, &sn, &cs);
-    }
+    const T kr = k * r, ikr = ir * kinv;
+    T sn, cs;
+    sincos_near(kr, &sn, &cs);
     // h0 = e^{ikr} / (i k r), h1 = h0 / (i k r) - ... (the first-order
     // spherical Hankel function), so that grad h0(kr) = -k h1 r / r
     const T h0r = sn * ikr, h0i = -cs * ikr;
@@ -288,15 +322,12 @@ k_p2p(EvalParams<T> p) {
           for (int c = 0; c < NA; c++) a[c] += (double)acc[c];
         }
       } else {
+        // the terms straight into the sums
         for (int j = gl; j < nt; j += g) {
-          // separation formed in FP64, the rest in T
           const T rx = (T)(x - tl.x[j]), ry = (T)(y - tl.y[j]), rz = (T)(z - tl.z[j]);
           const T r2 = rx * rx + ry * ry + rz * rz;
           if (!(r2 > rc2)) continue;
-          T acc[NA];
-          for (int c = 0; c < NA; c++) acc[c] = T(0);
-          p2p_pair<T, HELM, NT, POT, GRAD>(tl, j, rx, ry, rz, r2, k, kinv, hd, acc);
-          for (int c = 0; c < NA; c++) a[c] += (double)acc[c];
+          p2p_pair<T, HELM, NT, POT, GRAD>(tl, j, rx, ry, rz, r2, k, kinv, hd, (T*)a);
         }
       }
     }
