@@ -869,19 +869,25 @@ struct Solver : public wbfmm_b200_solver {
                                : lanes_supported<T, false>(x.Nin, x.Nout);
     const bool tiles_ok = helm ? tiles_supported<T, true>(x.Nin, x.Nout)
                                : tiles_supported<T, false>(x.Nin, x.Nout);
-    // (level 2 of an FP64 Laplace solve keeps the tiles: 8 targets of a type
-    // fill half of its columns' number pairs; 0.121 against 0.110 ms at p = 14)
+    // (level 2 of an FP64 Laplace solve keeps the tiles from order 10 on: 8
+    // targets of a type fill half of its columns' number pairs; 0.121 against
+    // 0.110 ms at p = 14)
     const bool cols_ok = helm ? cols_supported<T, true>(x.Nin, x.Nout)
                               : cols_supported<T, false>(x.Nin, x.Nout) &&
-                                    !(level == 2 && sizeof(T) == 8);
+                                    !(level == 2 && sizeof(T) == 8 && x.Nin >= 10);
     // automatic: lanes at the orders where their unrolled code wins, column
     // products above (tiles beyond their orders), the warp-per-target kernel
     // for what none covers.  Lanes / columns, ms on 32768 boxes: Helmholtz
-    // FP32 p = 6 1.37 / 2.90, p = 7 3.32 / 3.32 (4096 boxes 0.61 / 0.47);
-    // FP64 p = 6 4.13 / 5.84, p = 7 11.8 / 8.0; Laplace FP32 p = 8 1.25 / 2.11,
-    // p = 9 3.86 / 2.40; FP64 p = 8 4.11 / 4.42, p = 9 10.4 / 5.3; target lists
-    // change sides at the same orders
-    const int lanes_max = helm ? 6 : 8;
+    // FP32 p = 6 0.97 / 2.89, p = 7 3.32 / 3.32 (4096 boxes 0.44 / 0.47, 64 boxes
+    // 0.13 / 0.05); FP64 p = 6 3.08 / 5.84, p = 7 7.96 / 7.99 (64 boxes 0.16 /
+    // 0.06); Laplace FP32 p = 8 0.96 / 2.09, p = 9 3.04 / 2.40; FP64 p = 8 3.57 /
+    // 4.44, p = 9 8.59 / 5.29; target lists change sides at the same orders.
+    // The 64 boxes of level 2, whose columns are few, change earlier: FP64
+    // p = 5 0.090 / 0.056 (Helmholtz), p = 6 0.089 / 0.059 (Laplace); FP32
+    // Helmholtz p = 6 0.060 / 0.047
+    const int lanes_max = level > 2        ? (helm ? 6 : 8)
+                          : sizeof(T) == 8 ? 4
+                                           : (helm ? 5 : 8);
     bool use_tiles = false, use_lanes = false;
     const int he = helm ? helm_e[level] : 0;
     if (cfg.sparse) return m2l_sparse(level, x, he, tiles_ok, lanes_ok, lanes_max);
