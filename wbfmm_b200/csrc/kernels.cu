@@ -1,8 +1,8 @@
 // Leaf kernels: P2M and L2P.
 //
-//  P2M  one warp per leaf box; lanes take the box's sources 32 at a time and
-//       every coefficient contribution is reduced across the warp in a fixed
-//       order (deterministic), accumulating in shared memory.
+//  P2M  a group of 32 or 8 lanes per leaf box; lanes take the box's sources
+//       and every coefficient contribution is reduced across the group in a
+//       fixed order (deterministic), accumulating in shared memory.
 //  L2P  one thread per target.
 #include <cuda_runtime.h>
 
@@ -15,66 +15,66 @@
 
 namespace wbfmm {
 
-template <typename T>
-__device__ __forceinline__ T warp_sum(T v) {
+// Sums over the groups of G lanes of a warp of several values at once, by
+// transposing while reducing: after the exchanges across lanes G/2 (and G/4)
+// apart, each half (quarter) of a group carries one value, whose sum the
+// remaining steps form.  Two values: the first half of the group holds the
+// sum of a, the second of b; four: the quarters those of a, b, c, d (G = 32:
+// 6 shuffles instead of 20).
+template <int G, typename T>
+__device__ __forceinline__ T group_sum(T v) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-
-// Sums over the warp of several values at once, by transposing while
-// reducing: after the exchanges across lanes 16 (and 8) apart, each half
-// (quarter) of the warp carries one value, whose sum the remaining steps
-// form.  Two values: lanes 0-15 hold the sum of a, 16-31 of b (5 shuffles
-// instead of 10); four: lanes 0-7, 8-15, 16-23, 24-31 hold those of a, b,
-// c, d (6 shuffles instead of 20).
-template <typename T>
-__device__ __forceinline__ T warp_sum2(T a, T b, int lane) {
-  const bool hi = lane & 16;
-  T w = (hi ? b : a) + __shfl_xor_sync(0xffffffffu, hi ? a : b, 16);
+template <int G, typename T>
+__device__ __forceinline__ T group_sum2(T a, T b, int lane) {
+  const bool hi = lane & (G / 2);
+  T w = (hi ? b : a) + __shfl_xor_sync(0xffffffffu, hi ? a : b, G / 2);
 #pragma unroll
-  for (int o = 8; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+  for (int o = G / 4; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
   return w;
 }
-template <typename T>
-__device__ __forceinline__ T warp_sum4(T a, T b, T c, T d, int lane) {
-  const bool hi = lane & 16, q = lane & 8;
-  const T u = (hi ? c : a) + __shfl_xor_sync(0xffffffffu, hi ? a : c, 16);
-  const T v = (hi ? d : b) + __shfl_xor_sync(0xffffffffu, hi ? b : d, 16);
-  T w = (q ? v : u) + __shfl_xor_sync(0xffffffffu, q ? u : v, 8);
+template <int G, typename T>
+__device__ __forceinline__ T group_sum4(T a, T b, T c, T d, int lane) {
+  const bool hi = lane & (G / 2), q = lane & (G / 4);
+  const T u = (hi ? c : a) + __shfl_xor_sync(0xffffffffu, hi ? a : c, G / 2);
+  const T v = (hi ? d : b) + __shfl_xor_sync(0xffffffffu, hi ? b : d, G / 2);
+  T w = (q ? v : u) + __shfl_xor_sync(0xffffffffu, q ? u : v, G / 4);
 #pragma unroll
-  for (int o = 4; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+  for (int o = G / 8; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
   return w;
 }
 
-// the P2M kernel's emitters: each emission summed over the warp's points
-// (one per lane) into the warp's accumulator in shared memory; pairs of
-// emissions reduced together (warp_sum2 / warp_sum4), their sums added by
-// one lane of each half / quarter
-template <typename T>
+// the P2M kernel's emitters: each emission summed over the group's points
+// (one per lane) into the group's accumulator in shared memory; values that
+// come together are reduced together, their sums added by one lane of each
+// half / quarter
+template <typename T, int G>
 struct P2MEmitHelm {
   T* acc;
   int lane;
   __device__ __forceinline__ void operator()(int idx, T re, T im) const {
-    re = warp_sum(re); im = warp_sum(im);
-    if (lane == 0) { acc[2 * idx] += re; acc[2 * idx + 1] += im; }
+    const T w = group_sum2<G>(re, im, lane);
+    if ((lane & (G / 2 - 1)) == 0) acc[2 * idx + ((lane & (G / 2)) ? 1 : 0)] += w;
   }
   __device__ __forceinline__ void pair(int i1, T r1, T m1, int i2, T r2, T m2) const {
-    const T w = warp_sum4(r1, m1, r2, m2, lane);
-    if ((lane & 7) == 0) acc[2 * ((lane & 16) ? i2 : i1) + ((lane & 8) ? 1 : 0)] += w;
+    const T w = group_sum4<G>(r1, m1, r2, m2, lane);
+    if ((lane & (G / 4 - 1)) == 0)
+      acc[2 * ((lane & (G / 2)) ? i2 : i1) + ((lane & (G / 4)) ? 1 : 0)] += w;
   }
 };
-template <typename T>
+template <typename T, int G>
 struct P2MEmitLap {
   T* acc;
   int lane;
   __device__ __forceinline__ void operator()(int idx, T v) const {
-    v = warp_sum(v);
-    if (lane == 0) acc[idx] += v;
+    v = group_sum<G>(v);
+    if ((lane & (G - 1)) == 0) acc[idx] += v;
   }
   __device__ __forceinline__ void pair(int i1, T v1, int i2, T v2) const {
-    const T w = warp_sum2(v1, v2, lane);
-    if ((lane & 15) == 0) acc[(lane & 16) ? i2 : i1] += w;
+    const T w = group_sum2<G>(v1, v2, lane);
+    if ((lane & (G / 2 - 1)) == 0) acc[(lane & (G / 2)) ? i2 : i1] += w;
   }
 };
 
@@ -121,11 +121,20 @@ constexpr int kFixedOrder = 14;   // P2M / L2P order with a compile-time instant
 // SROWS: recursion rows in shared memory (else per-thread local arrays);
 // NC > 0: the expansion order fixed at compile time (p.N == NC), the rows
 // in a per-thread array whose every index the unrolled recursion knows, so
-// that they stay in registers
-template <typename T, bool HELM, bool SROWS, int NC = 0>
-__global__ void k_p2m(P2MParams<T> p, int legt) {
+// that they stay in registers.
+// A warp takes 32 / G boxes, G lanes each: with a few points per leaf a whole
+// warp per box leaves most lanes idle.  The grid is what the SMs hold, each
+// CTA walking over the boxes, so that the recursion constants (square roots
+// and divisions) are formed once per CTA and not once per four boxes (the
+// 262144 leaves of 1e6 points, FP64 Helmholtz p = 6: 2.88 ms with a CTA per
+// four leaves and a warp per leaf, 0.84 so).
+// share (G = 32): the warps of a CTA share a box and their sums are added in
+// warp order, for trees of fewer boxes than the SMs have warps.
+template <typename T, bool HELM, bool SROWS, int NC, int G>
+__global__ void k_p2m(P2MParams<T> p, int legt, int share) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int NG = 32 / G;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gl = lane & (G - 1);
   const int nw = blockDim.x >> 5;
   // Legendre recursion constants of degrees <= N + 2, once per CTA
   const int LW = (NC > 0 ? NC : p.N) + 3;
@@ -134,10 +143,6 @@ __global__ void k_p2m(P2MParams<T> p, int legt) {
     leg_table_fill(lt, LW - 1, threadIdx.x, blockDim.x);
     __syncthreads();
   }
-  // the box's storage index, and (sparse storage) its Morton index
-  const int64_t cb = (int64_t)blockIdx.x * nw + warp;
-  if (cb >= p.nbox) return;   // whole warp leaves; no block barriers below
-  const int64_t b = p.glist ? (((int64_t)p.glist[cb >> 3] << 3) | (cb & 7)) : cb;
   const int N = NC > 0 ? NC : p.N;
   const int nc = ncoef(N);
   const int w = HELM ? 2 : 1;
@@ -146,67 +151,87 @@ __global__ void k_p2m(P2MParams<T> p, int legt) {
   T loc[NC > 0 ? 2 * (NC + kRowPad) : (SROWS ? 1 : 2 * kPtMax)];
   const Scratch<T> sc = SROWS && NC == 0 ? Scratch<T>{rows + threadIdx.x, RL, (int)blockDim.x}
                                          : Scratch<T>{loc, RL, 1};
-  T* acc = rows + (SROWS && NC == 0 ? p2m_rows() * RL * blockDim.x : 0) + (size_t)warp * nc * w;
-  for (int c = lane; c < nc * w; c += 32) acc[c] = T(0);
-  __syncwarp();
-  const uint32_t cnt = p.box_n[b], start = p.box_i[b];
-  if (cnt > 0) {
-    double cd[3];
-    box_centre(b, p.x0, p.y0, p.z0, p.wb, cd);
-    // source position relative to the box centre, formed in FP64
-    const T xc[3] = {T(0), T(0), T(0)};
-    for (uint32_t base = 0; base < cnt; base += 32) {
-      const uint32_t t = base + lane;
-      const bool act = t < cnt;
-      const uint32_t s = start + (act ? t : 0);
-      T xs[3] = {act ? (T)(p.x[s] - cd[0]) : T(0),
-                 act ? (T)(p.y[s] - cd[1]) : T(0),
-                 act ? (T)(p.z[s] - cd[2]) : T(0)};
-      auto expand = [&](const auto& leg) {
-        if (HELM) {
-          const P2MEmitHelm<T> emit{acc, lane};
-          if (p.q) {
-            T qr = act ? p.q[2 * s] : T(0), qi = act ? p.q[2 * s + 1] : T(0);
-            p2m_helmholtz<T>(N, p.k, xc, xs, qr, qi, emit, leg, sc);
+  T* acc = rows + (SROWS && NC == 0 ? p2m_rows() * RL * blockDim.x : 0) +
+           (size_t)(warp * NG + lane / G) * nc * w;
+#pragma unroll 1
+  for (int64_t c0 = share ? (int64_t)blockIdx.x : ((int64_t)blockIdx.x * nw + warp) * NG; c0 < p.nbox;
+       c0 += share ? (int64_t)gridDim.x : (int64_t)gridDim.x * nw * NG) {
+    // the box's storage index, and (sparse storage) its Morton index
+    const int64_t cb = c0 + lane / G;
+    const bool in = cb < p.nbox;
+    const int64_t b = !in ? 0 : p.glist ? (((int64_t)p.glist[cb >> 3] << 3) | (cb & 7)) : cb;
+    const uint32_t cnt = in ? p.box_n[b] : 0, start = in ? p.box_i[b] : 0;
+    const uint32_t most = NG == 1 ? cnt : __reduce_max_sync(0xffffffffu, cnt);
+    if (most > 0) {
+      for (int c = gl; c < nc * w; c += G) acc[c] = T(0);
+      __syncwarp();
+      double cd[3];
+      box_centre(b, p.x0, p.y0, p.z0, p.wb, cd);
+      // source position relative to the box centre, formed in FP64
+      const T xc[3] = {T(0), T(0), T(0)};
+      for (uint32_t base = share ? warp * G : 0; base < most; base += share ? nw * G : G) {
+        const uint32_t t = base + gl;
+        const bool act = t < cnt;
+        const uint32_t s = act ? start + t : 0;
+        T xs[3] = {act ? (T)(p.x[s] - cd[0]) : T(0),
+                   act ? (T)(p.y[s] - cd[1]) : T(0),
+                   act ? (T)(p.z[s] - cd[2]) : T(0)};
+        auto expand = [&](const auto& leg) {
+          if (HELM) {
+            const P2MEmitHelm<T, G> emit{acc, lane};
+            if (p.q) {
+              T qr = act ? p.q[2 * s] : T(0), qi = act ? p.q[2 * s + 1] : T(0);
+              p2m_helmholtz<T>(N, p.k, xc, xs, qr, qi, emit, leg, sc);
+            }
+            if (p.dip) {
+              T dr = act ? p.dip[2 * s] : T(0), di = act ? p.dip[2 * s + 1] : T(0);
+              T nrm[3] = {act ? p.nx[s] : T(0), act ? p.ny[s] : T(0),
+                          act ? p.nz[s] : T(1)};
+              p2m_helmholtz_dipole<T>(N, p.k, xc, xs, nrm, dr, di, emit, leg, sc);
+            }
+          } else {
+            const P2MEmitLap<T, G> emit{acc, lane};
+            if (p.q) {
+              T qv = act ? p.q[s] : T(0);
+              p2m_laplace<T>(N, xc, xs, qv, emit, leg, sc);
+            }
+            if (p.dip) {
+              T dv = act ? p.dip[s] : T(0);
+              T nrm[3] = {act ? p.nx[s] : T(0), act ? p.ny[s] : T(0),
+                          act ? p.nz[s] : T(1)};
+              p2m_laplace_dipole<T>(N, xc, xs, nrm, dv, emit, leg, sc);
+            }
           }
-          if (p.dip) {
-            T dr = act ? p.dip[2 * s] : T(0), di = act ? p.dip[2 * s + 1] : T(0);
-            T nrm[3] = {act ? p.nx[s] : T(0), act ? p.ny[s] : T(0),
-                        act ? p.nz[s] : T(1)};
-            p2m_helmholtz_dipole<T>(N, p.k, xc, xs, nrm, dr, di, emit, leg, sc);
-          }
-        } else {
-          const P2MEmitLap<T> emit{acc, lane};
-          if (p.q) {
-            T qv = act ? p.q[s] : T(0);
-            p2m_laplace<T>(N, xc, xs, qv, emit, leg, sc);
-          }
-          if (p.dip) {
-            T dv = act ? p.dip[s] : T(0);
-            T nrm[3] = {act ? p.nx[s] : T(0), act ? p.ny[s] : T(0),
-                        act ? p.nz[s] : T(1)};
-            p2m_laplace_dipole<T>(N, xc, xs, nrm, dv, emit, leg, sc);
-          }
-        }
-      };
-      if (legt) expand(LegTab<T>{lt, LW});
-      else expand(LegDirect<T>());
-    }
-  }
-  __syncwarp();
-  for (int c = lane; c < nc; c += 32) {
-    int64_t o = layout_off(cb, c, nc);
-    if (HELM) {
-      if (p.accumulate) {
-        p.mps[2 * o] += acc[2 * c];
-        p.mps[2 * o + 1] += acc[2 * c + 1];
-      } else {
-        p.mps[2 * o] = acc[2 * c];
-        p.mps[2 * o + 1] = acc[2 * c + 1];
+        };
+        if (legt) expand(LegTab<T>{lt, LW});
+        else expand(LegDirect<T>());
       }
-    } else {
-      if (p.accumulate) p.mps[o] += acc[c]; else p.mps[o] = acc[c];
+      __syncwarp();
     }
+    if (share) {
+      if (most > 0) {
+        __syncthreads();     // (the box is the CTA's)
+        if (warp == 0)
+          for (int c = lane; c < nc * w; c += 32)
+            for (int u = 1; u < nw; u++) acc[c] += acc[c + u * nc * w];
+        __syncwarp();
+      }
+      if (warp) {
+        if (most > 0) __syncthreads();
+        continue;
+      }
+    }
+    // (a box without points beside one with points holds zeros)
+    for (int c = gl; in && c < nc; c += G) {
+      const int64_t o = layout_off(cb, c, nc);
+      for (int u = 0; u < w; u++) {
+        const T v = most > 0 ? acc[w * c + u] : T(0);
+        if (p.accumulate) p.mps[w * o + u] += v;
+        else p.mps[w * o + u] = v;
+      }
+    }
+    if (share && most > 0) __syncthreads();
+    else __syncwarp();
   }
 }
 
@@ -216,24 +241,39 @@ int launch_p2m(const P2MParams<T>& p, cudaStream_t s) {
   const int nw = 4;
   const size_t leg = leg_table_bytes<T>(p.N);
   const size_t rows = p2m_row_bytes<T>(p.N, nw * 32);
-  const bool srows = rows <= kRowSmemMax;
-  size_t smem = leg + (srows ? rows : 0) + sizeof(T) * (size_t)nw * ncoef(p.N) * (HELM ? 2 : 1);
-  unsigned grid = (unsigned)((p.nbox + nw - 1) / nw);
+  const size_t one = sizeof(T) * (size_t)nw * ncoef(p.N) * (HELM ? 2 : 1);   // a box per warp
+  // leaves of up to 12 points on average: four boxes per warp, while their
+  // accumulators leave room for a second CTA; not where most boxes are empty
+  // and the others full (surface points, 33 per occupied leaf: 4.2 ms against
+  // 3.1)
+  const bool few = !p.skewed && p.npts <= 12 * p.nbox && leg + rows + 4 * one <= 100 * 1024;
+  const bool share = !few && p.nbox <= 148 * 8 && p.npts > 48 * p.nbox;
+  auto go = [&](auto srows, auto nc, auto group) -> int {
+    constexpr bool SR = decltype(srows)::value;
+    constexpr int NC = decltype(nc)::value, G = decltype(group)::value;
+    const size_t smem = leg + (SR ? rows : 0) + one * (32 / G);
+    if (smem > 48 * 1024) WBFMM_SMEM(smem, k_p2m<T, HELM, SR, NC, G>);
+    // at most 8 CTAs per SM: about what registers and shared memory hold
+    const int64_t need = (p.nbox + nw * (32 / G) - 1) / (nw * (32 / G));
+    const unsigned grid = (unsigned)(need < 148 * 8 ? need : 148 * 8);
+    k_p2m<T, HELM, SR, NC, G><<<share ? (unsigned)p.nbox : grid, nw * 32, smem, s>>>(
+        p, leg ? 1 : 0, share ? 1 : 0);
+    return 0;
+  };
+  const std::integral_constant<int, 0> any;
+  const std::integral_constant<int, 32> whole;
+  const std::integral_constant<int, 8> eighth;
+  const std::true_type yes;
+  const std::false_type no;
   // the serving orders' leaf expansions: rows in registers (not for FP64
   // Helmholtz, whose unrolled recursion exceeds the register file)
   constexpr bool kFixedOk = !(HELM && sizeof(T) == 8);
-  if (kFixedOk && p.N == kFixedOrder) {
-    if constexpr (kFixedOk) {
-      const size_t sm = leg + sizeof(T) * (size_t)nw * ncoef(p.N) * (HELM ? 2 : 1);
-      if (sm > 48 * 1024) WBFMM_SMEM(sm, k_p2m<T, HELM, false, kFixedOrder>);
-      k_p2m<T, HELM, false, kFixedOrder><<<grid, nw * 32, sm, s>>>(p, leg ? 1 : 0);
-    }
-  } else if (srows) {
-    if (smem > 48 * 1024) WBFMM_SMEM(smem, k_p2m<T, HELM, true>);
-    k_p2m<T, HELM, true><<<grid, nw * 32, smem, s>>>(p, leg ? 1 : 0);
+  if (few) {
+    WBFMM_TRY_K(rows <= kRowSmemMax ? go(yes, any, eighth) : go(no, any, eighth));
+  } else if (kFixedOk && p.N == kFixedOrder) {
+    if constexpr (kFixedOk) WBFMM_TRY_K(go(no, std::integral_constant<int, kFixedOrder>(), whole));
   } else {
-    if (smem > 48 * 1024) WBFMM_SMEM(smem, k_p2m<T, HELM, false>);
-    k_p2m<T, HELM, false><<<grid, nw * 32, smem, s>>>(p, leg ? 1 : 0);
+    WBFMM_TRY_K(rows <= kRowSmemMax ? go(yes, any, whole) : go(no, any, whole));
   }
   WBFMM_CUDA(cudaGetLastError());
   return 0;

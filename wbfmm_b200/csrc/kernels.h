@@ -39,6 +39,8 @@ struct OpTables {
 template <typename T>
 struct P2MParams {
   int64_t nbox;       // boxes at the leaf level
+  int64_t npts;       // sources in them
+  int skewed;         // most boxes may be empty (dense storage with skip_empty)
   int level, N;
   double x0, y0, z0, wb;
   T k;

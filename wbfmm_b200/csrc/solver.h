@@ -789,6 +789,8 @@ struct Solver : public wbfmm_b200_solver {
     WBFMM_TRY(prepare_sparse());
     P2MParams<T> p;
     p.nbox = (int64_t)1 << (3 * depth);
+    p.npts = nsrc;
+    p.skewed = cfg.skip_empty && !cfg.sparse;
     p.level = depth; p.N = cfg.order_s[depth];
     p.x0 = cfg.x0[0]; p.y0 = cfg.x0[1]; p.z0 = cfg.x0[2]; p.wb = width(depth);
     p.k = (T)cfg.k;
