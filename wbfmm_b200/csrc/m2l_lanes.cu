@@ -424,37 +424,24 @@ k_m2l_lanes(LanesParams<T> p, OpTables<T> t) {
     const int64_t cs = p.boxmajor ? 1 : lstride;
     const T2* src = (const T2*)p.lin_raw + (int64_t)sg * V * lstride + (p.boxmajor ? col * V : col);
     if constexpr (HELM) {
-      // source phases: E = c S+ - s S'', O'' = c S'' + s S+
-#pragma unroll
-      for (int n = 0; n <= P; n++) {
-        w[le_row(n, 0)] = __ldg(src + (int64_t)le_row(n, 0) * cs);
+      // source phases, E = c S+ - s S'', O'' = c S'' + s S+, and the forward
+      // rotation of each degree, from the source to the working vector
+      lane_for<0, P>([&](auto nn) {
+        constexpr int n = decltype(nn)::value;
+        T2 in[n + 1], io[n > 0 ? n : 1];
+        in[0] = __ldg(src + (int64_t)le_row(n, 0) * cs);
 #pragma unroll
         for (int m = 1; m <= n; m++) {
           const T2 e = __ldg(src + (int64_t)le_row(n, m) * cs);
           const T2 o = __ldg(src + (int64_t)lo_row(P, n, m) * cs);
           const T c = sech[2 * m], sn = sech[2 * m + 1];
-          T2 x, y;
-          x.x = c * e.x - sn * o.x; x.y = c * e.y - sn * o.y;
-          y.x = c * o.x + sn * e.x; y.y = c * o.y + sn * e.y;
-          w[le_row(n, m)] = x;
-          w[lo_row(P, n, m)] = y;
+          in[m].x = c * e.x - sn * o.x; in[m].y = c * e.y - sn * o.y;
+          io[m - 1].x = c * o.x + sn * e.x; io[m - 1].y = c * o.y + sn * e.y;
         }
-        cfence();
-      }
-      // forward rotation per degree, in place
-      lane_for<0, P>([&](auto nn) {
-        constexpr int n = decltype(nn)::value;
-        T2 in[n + 1];
-#pragma unroll
-        for (int m = 0; m <= n; m++) in[m] = w[le_row(n, m)];
         lane_block<n + 1, n + 1>(ops + lane_h<T>(n), in, [&](int i, T2 v) { w[le_row(n, i)] = v; });
-        if constexpr (n > 0) {
-          T2 io[n];
-#pragma unroll
-          for (int m = 0; m < n; m++) io[m] = w[lo_row(P, n, m + 1)];
+        if constexpr (n > 0)
           lane_block<n, n>(ops + lane_h<T>(n) + (n + 1) * lane_pad<T>(n + 1), io,
                            [&](int i, T2 v) { w[lo_row(P, n, i + 1)] = v; });
-        }
         cfence();
       });
       // coaxial (S|R) per order, both parts with one read of the table
@@ -516,23 +503,11 @@ k_m2l_lanes(LanesParams<T> p, OpTables<T> t) {
     } else {
       // Laplace, half vectors (m >= 0; negative m are conjugates): x the even
       // parts, y the odd ones
-#pragma unroll
-      for (int n = 0; n <= P; n++) {
-#pragma unroll
-        for (int m = 0; m <= n; m++) {
-          T2 v = __ldg(src + (int64_t)hidx(n, m) * cs);
-          w[hidx(n, m)] = cm(v, sech[2 * m], sech[2 * m + 1]);
-        }
-        cfence();
-      }
       // (E, O'') of row nu from the degree's vector
-      auto rotate = [&](auto nn, auto out) {
+      auto rotate = [&](auto nn, const auto& in, auto out) {
         constexpr int n = decltype(nn)::value, RE = lane_pad<T>(n + 1), RO = lane_pad<T>(n > 0 ? n : 1);
         const T* te = ops + lane_h<T>(n);
         const T* to = te + (n + 1) * RE;
-        T2 in[n + 1];
-#pragma unroll
-        for (int m = 0; m <= n; m++) in[m] = w[hidx(n, m)];
 #pragma unroll
         for (int nu = 0; nu <= n; nu++) {
           LaneRow<T, n + 1> re;
@@ -555,7 +530,11 @@ k_m2l_lanes(LanesParams<T> p, OpTables<T> t) {
       };
       lane_for<0, P>([&](auto nn) {
         constexpr int n = decltype(nn)::value;
-        rotate(nn, [&](int nu, T2 o) { w[hidx(n, nu)] = o; });
+        T2 in[n + 1];
+#pragma unroll
+        for (int m = 0; m <= n; m++)
+          in[m] = cm(T2(__ldg(src + (int64_t)hidx(n, m) * cs)), sech[2 * m], sech[2 * m + 1]);
+        rotate(nn, in, [&](int nu, T2 o) { w[hidx(n, nu)] = o; });
       });
       lane_for<0, P>([&](auto mm) {
         constexpr int m = decltype(mm)::value, L = P + 1 - m, RS = lane_pad<T>(L);
@@ -571,7 +550,10 @@ k_m2l_lanes(LanesParams<T> p, OpTables<T> t) {
       });
       lane_for<0, P>([&](auto nn) {
         constexpr int n = decltype(nn)::value;
-        rotate(nn, [&](int nu, T2 o) {
+        T2 in[n + 1];
+#pragma unroll
+        for (int m = 0; m <= n; m++) in[m] = w[hidx(n, m)];
+        rotate(nn, in, [&](int nu, T2 o) {
           const T er = sech[2 * nu], ei = sech[2 * nu + 1];
           T2 a = acc[hidx(n, nu) * 32];
           a.x += er * o.x + ei * o.y;
