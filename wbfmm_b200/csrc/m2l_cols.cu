@@ -342,7 +342,7 @@ __global__ void k_cols_rotations(const double* __restrict__ H, int64_t hstride,
 template <typename T, bool HELM>
 __global__ void k_cols_planes(const T* __restrict__ arr, int level, int N, int scale_e,
                               int64_t groups, int64_t ncols, bool boxmajor,
-                              T* __restrict__ lin) {
+                              const uint32_t* __restrict__ src_n, T* __restrict__ lin) {
   typedef typename P2<T>::t T2;
   const int64_t pp = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (pp >= ncols) return;
@@ -366,6 +366,7 @@ __global__ void k_cols_planes(const T* __restrict__ arr, int level, int N, int s
   const int64_t rs = boxmajor ? 1 : ncols, first = boxmajor ? pp * V : pp;
 #pragma unroll
   for (int tau = 0; tau < 8; tau++) {
+    if (src_n && !(in && src_n[(P << 3) | tau])) continue;   // never read
     if (HELM) {
       T2 a, b;
       a.x = a.y = b.x = b.y = T(0);
@@ -1163,11 +1164,11 @@ ColsWork cols_work(int P, int level) {
 
 template <typename T, bool HELM>
 int cols_planes(const T* arr, int level, int N, int scale_e, int64_t groups, void* lin,
-                cudaStream_t s, bool boxmajor) {
+                cudaStream_t s, bool boxmajor, const uint32_t* src_n) {
   const int64_t npx = (1 << (level - 1)) + 2;
   const int64_t ncols = groups >= 0 ? groups + 1 : npx * npx * npx;
   k_cols_planes<T, HELM><<<dim3((unsigned)((ncols + 127) / 128), o_base(N)), 128, 0, s>>>(
-      arr, level, N, scale_e, groups, ncols, boxmajor, (T*)lin);
+      arr, level, N, scale_e, groups, ncols, boxmajor, src_n, (T*)lin);
   WBFMM_CUDA(cudaGetLastError());
   return 0;
 }
@@ -1198,7 +1199,8 @@ int launch_m2l_cols(const LanesParams<T>& p, const OpTables<T>& t, T* table, voi
 #define WBFMM_COLS_INST(T, H)                                                              \
   template bool cols_supported<T, H>(int, int);                                            \
   template ColsWork cols_work<T, H>(int, int);                                             \
-  template int cols_planes<T, H>(const T*, int, int, int, int64_t, void*, cudaStream_t, bool); \
+  template int cols_planes<T, H>(const T*, int, int, int, int64_t, void*, cudaStream_t, bool, \
+                                 const uint32_t*);                                         \
   template int launch_m2l_cols<T, H>(const LanesParams<T>&, const OpTables<T>&, T*, void*, \
                                      cudaStream_t);
 WBFMM_COLS_INST(double, true)

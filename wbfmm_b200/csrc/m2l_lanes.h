@@ -131,10 +131,12 @@ int build_cols_rotations(const double* H, int64_t hstride, int nth, int L, T* he
 // level array (Layout L), degree n scaled by 2^(scale_e n): lin[tau][row][pp]
 // over the padded parent grid (groups < 0; lanes_lin_bytes), or over the
 // groups stored and a zero column (lanes_lin_groups_bytes); boxmajor:
-// lin[tau][pp][row]
+// lin[tau][pp][row]; with src_n (dense storage, the level's source counts) the
+// boxes without sources are left out (kernels with a source mask do not read
+// them)
 template <typename T, bool HELM>
 int cols_planes(const T* arr, int level, int N, int scale_e, int64_t groups, void* lin,
-                cudaStream_t s, bool boxmajor = false);
+                cudaStream_t s, bool boxmajor = false, const uint32_t* src_n = nullptr);
 template <typename T, bool HELM>
 int launch_m2l_cols(const LanesParams<T>& p, const OpTables<T>& t, T* table, void* tasks,
                     cudaStream_t s);

@@ -965,7 +965,8 @@ struct Solver : public wbfmm_b200_solver {
       // (box-major for target lists)
       const bool boxmajor = x.tmask && act[level].p;
       WBFMM_TRY(lin.alloc(lanes_lin_bytes(level, x.Nin, helm, sizeof(T))));
-      WBFMM_TRY((helm ? cols_planes<T, true>(x.cin, level, x.Nin, 0, -1, lin.p, stream, boxmajor)
+      WBFMM_TRY((helm ? cols_planes<T, true>(x.cin, level, x.Nin, 0, -1, lin.p, stream, boxmajor,
+                                              x.tmask ? x.src_n : nullptr)
                       : lanes_to_lin<T, false>(x.cin, level, x.Nin, x.lap_e, lin.p, stream,
                                                boxmajor)));
       LanesParams<T> lp;
@@ -1035,8 +1036,9 @@ struct Solver : public wbfmm_b200_solver {
     const int64_t G = cfg.sparse ? ngroups[level] : -1;
     WBFMM_TRY(lin.alloc(cfg.sparse ? lanes_lin_groups_bytes(G, x.Nin, helm, sizeof(T))
                                    : lanes_lin_bytes(level, x.Nin, helm, sizeof(T))));
-    WBFMM_TRY((helm ? cols_planes<T, true>(x.cin, level, x.Nin, he, G, lin.p, stream)
-                    : cols_planes<T, false>(x.cin, level, x.Nin, x.lap_e, G, lin.p, stream)));
+    const uint32_t* sn = x.tmask && !cfg.sparse ? x.src_n : nullptr;
+    WBFMM_TRY((helm ? cols_planes<T, true>(x.cin, level, x.Nin, he, G, lin.p, stream, false, sn)
+                    : cols_planes<T, false>(x.cin, level, x.Nin, x.lap_e, G, lin.p, stream, false, sn)));
     lp.lin_raw = lin.p;
     if (cfg.sparse) {
       WBFMM_TRY(pmap.alloc(source_mask_bytes(level) / 8));
