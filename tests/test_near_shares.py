@@ -1,0 +1,73 @@
+"""The near field alone: sources and targets in one leaf and its neighbour, so
+that no expansion reaches a target.  FP32 terms are formed two at a time and a
+tree of few leaves shares a leaf's targets between CTAs; here at lone, odd and
+tile-crossing source counts, and at target counts of one and of several shares."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from wbfmm_b200 import engine
+
+pytestmark = pytest.mark.gpu
+
+
+def _direct(problem, k, xs, q, nrm, d, xt):
+    r = xt[:, None] - xs[None]
+    R = np.linalg.norm(r, axis=2)
+    on = R > 1e-6
+    R = np.where(on, R, 1.0)
+    if problem == engine.LAPLACE:
+        G, G1, G2 = 1 / R, -1 / R**2, 2 / R**3
+    else:
+        e = np.exp(1j * k * R) / (1j * k)
+        G, G1 = e / R, e * (1j * k / R - 1 / R**2)
+        G2 = e * (-k * k / R - 2j * k / R**2 + 2 / R**3)
+    G, G1, G2 = (np.where(on, a, 0.0) / (4 * np.pi) for a in (G, G1, G2))
+    u = r / R[..., None]
+    pot, grad = G @ q, np.einsum("ts,tsc,s->tc", G1, u, q)
+    if d is not None:        # n . grad over the sources (Laplace), the targets (Helmholtz)
+        d = -d if problem == engine.LAPLACE else d
+        nu = np.einsum("tsc,sc->ts", u, nrm)
+        pot = pot + (G1 * nu) @ d
+        g = (G2 * nu)[..., None] * u + (G1 / R)[..., None] * (nrm[None] - nu[..., None] * u)
+        grad = grad + np.einsum("tsc,s->tc", g, d)
+    return pot, grad
+
+
+# FP32: a term is a dozen operations of half an ulp (6e-8) each, cubed 1/r
+# tripling its own: below 2e-6 of the term, and no sum is larger than its terms
+@pytest.mark.parametrize("precision,tol", [(engine.FP64, 1e-12), (engine.FP32, 5e-6)])
+@pytest.mark.parametrize("problem", [engine.LAPLACE, engine.HELMHOLTZ])
+@pytest.mark.parametrize("ns,nt", [(1, 1), (2, 9), (7, 40), (127, 511), (129, 520), (128, 1100),
+                                   (301, 3000)])
+@pytest.mark.parametrize("dipoles", [False, True])
+def test_near(gpu_lib, problem, precision, tol, ns, nt, dipoles):
+    rng = np.random.default_rng(ns + nt)
+    k = 6.0 if problem == engine.HELMHOLTZ else 0.0
+    xs, xt = rng.uniform(0.01, 0.24, (ns, 3)), rng.uniform(0.01, 0.24, (nt, 3))
+    xs[:, 0] += 0.255 * (np.arange(ns) % 2)              # the leaf and its neighbour
+    same = min(ns, nt) // 2
+    xt[:same] = xs[:same]                                # pairs within the cutoff
+    shape = (ns, 2) if problem == engine.HELMHOLTZ else (ns, 1)
+    q, d = rng.uniform(0.5, 1.0, shape), rng.uniform(0.5, 1.0, shape)
+    nrm = rng.standard_normal((ns, 3))
+    nrm /= np.linalg.norm(nrm, axis=1, keepdims=True)
+    orders = [0, 8, 8]
+    cfg = engine.SolverConfig(problem, 2, orders, list(orders), k, (-0.51,) * 3, 1.02, precision,
+                              engine.POTENTIAL | engine.GRADIENT)
+    with engine.Solver(cfg) as s:
+        s.set_sources(xs, nrm if dipoles else None)
+        s.set_strengths(q.ravel(), d.ravel() if dipoles else None)
+        s.set_targets(xt)
+        s.run()
+        pot, grad = s.field()
+
+    def whole(a):
+        return a[..., 0] + 1j * a[..., 1] if problem == engine.HELMHOLTZ else a[..., 0]
+    P, G = _direct(problem, k, xs, whole(q), nrm, whole(d) if dipoles else None, xt)
+    got_p, got_g = np.asarray(pot).ravel(), np.asarray(grad).ravel()
+    if problem == engine.HELMHOLTZ:
+        got_p, got_g = got_p[0::2] + 1j * got_p[1::2], got_g[0::2] + 1j * got_g[1::2]
+    assert np.linalg.norm(got_p - P) <= tol * np.linalg.norm(P)
+    assert np.linalg.norm(got_g - G.ravel()) <= tol * np.linalg.norm(G)

@@ -55,6 +55,7 @@
 #include <mutex>
 
 #include "engine.h"
+#include "f32x2.cuh"
 #include "kernels.h"
 #include "m2l_lanes.h"
 #include "tables.h"
@@ -420,41 +421,19 @@ __device__ __forceinline__ void cpa_wait() { asm volatile("cp.async.wait_all;\n"
 // (fma.rn.f32x2: both numbers in one instruction, halving the issue slots
 // the products take), FP64 pairs as double2.
 template <typename T> struct Col;
-template <> struct Col<float> { typedef unsigned long long t; };
+template <> struct Col<float> { typedef f32x2 t; };
 template <> struct Col<double> { typedef double2 t; };
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 both(float h) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(h));
-  return r;
-}
+using wbfmm::both;
 __device__ __forceinline__ double both(double h) { return h; }
-__device__ __forceinline__ void mac(f32x2& a, f32x2 h, f32x2 x) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(a) : "l"(h), "l"(x));
-}
+__device__ __forceinline__ void mac(f32x2& a, f32x2 h, f32x2 x) { a = fma2(h, x, a); }
 __device__ __forceinline__ void mac(double2& a, double h, const double2& x) {
   a.x = fma(h, x.x, a.x);
   a.y = fma(h, x.y, a.y);
 }
-__device__ __forceinline__ f32x2 mul(f32x2 h, f32x2 x) {
-  f32x2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(h), "l"(x));
-  return r;
-}
+__device__ __forceinline__ f32x2 mul(f32x2 h, f32x2 x) { return mul2(h, x); }
 __device__ __forceinline__ double2 mul(double h, const double2& x) {
   return make_double2(h * x.x, h * x.y);
 }
-__device__ __forceinline__ float2 pair(f32x2 a) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
-  return r;
-}
-__device__ __forceinline__ f32x2 packed(const float2& a) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
-  return r;
-}
-
 // where column col of a row with (n + m) & 3 = g stands in the row's NC:
 // FP32 rows of odd g hold their 64-byte halves exchanged, FP64 rows their
 // 32-byte quarters in the order j ^ g and, for odd g, each quarter's two

@@ -6,6 +6,7 @@
 
 #include "engine.h"
 #include "expand.cuh"
+#include "f32x2.cuh"
 #include "kernels.h"
 #include "translate.cuh"
 
@@ -190,6 +191,101 @@ __device__ __forceinline__ void p2p_pair(const P2PTile<T, HELM, NT>& tl, int j, 
   }
 }
 
+// sincos_near of both numbers of a pair: sin and cos of r packed (the same
+// reduction, the quadrant from adding 1.5 x 2^23, the same series), the
+// quadrant's swap and signs one by one
+__device__ __forceinline__ void sincos_near(f32x2 x, f32x2* sp, f32x2* cp) {
+  const f32x2 t = fma2(x, both(0.636619772367581343f), both(12582912.0f));
+  const f32x2 q = add2(t, both(-12582912.0f));
+  f32x2 r = fma2(q, both(-1.57079637050628662109375f), x);
+  r = fma2(q, both(4.37113900018624283e-8f), r);
+  const f32x2 r2 = mul2(r, r);
+  f32x2 ps = fma2(r2, both(2.75573192239858907e-6f), both(-1.98412698412698413e-4f));
+  ps = fma2(r2, ps, both(8.33333333333333333e-3f));
+  ps = fma2(r2, ps, both(-1.66666666666666667e-1f));
+  const float2 sn = pair(fma2(mul2(r, r2), ps, r));
+  f32x2 pc = fma2(r2, both(-2.75573192239858907e-7f), both(2.48015873015873016e-5f));
+  pc = fma2(r2, pc, both(-1.38888888888888889e-3f));
+  pc = fma2(r2, pc, both(4.16666666666666667e-2f));
+  pc = fma2(r2, pc, both(-0.5f));
+  const float2 cn = pair(fma2(r2, pc, both(1.0f)));
+  const float2 tf = pair(t);
+  auto turn = [](float tq, float s, float c, float* so, float* co) {
+    const int n = __float_as_int(tq);        // low bits: the quadrant
+    const float a = (n & 1) ? c : s, b = (n & 1) ? s : c;
+    *so = __int_as_float(__float_as_int(a) ^ ((n & 2) << 30));
+    *co = __int_as_float(__float_as_int(b) ^ (((n + 1) & 2) << 30));
+  };
+  float2 so, co;
+  turn(tf.x, sn.x, cn.x, &so.x, &co.x);
+  turn(tf.y, sn.y, cn.y, &so.y, &co.y);
+  *sp = packed(so);
+  *cp = packed(co);
+}
+
+// p2p_pair (monopoles, cutoff masked) of tile entries j0 and j1, the terms
+// two at a time in packed arithmetic (f32x2.cuh) and then added one after
+// the other: the operations and the order of sums of two calls of p2p_pair.
+// second: false for a lone entry j0 (1/r of the other is then 0).
+// t: the target's coordinates, each hi and lo
+template <bool HELM, int NT, bool POT, bool GRAD>
+__device__ __forceinline__ void p2p_two(const P2PTile<float, HELM, NT>& tl, int j0, int j1,
+                                        bool second, const f32x2 (&t)[3], float rc2, f32x2 k,
+                                        f32x2 kinv, float* acc) {
+  const f32x2 m1 = both(-1.0f);
+  auto sep = [&](const double* a, f32x2 tc) {
+    const f32x2* c = reinterpret_cast<const f32x2*>(a);
+    const float2 d0 = pair(fma2(c[j0], m1, tc)), d1 = pair(fma2(c[j1], m1, tc));
+    return packed(make_float2(d0.x + d0.y, d1.x + d1.y));
+  };
+  const f32x2 rx = sep(tl.x, t[0]), ry = sep(tl.y, t[1]), rz = sep(tl.z, t[2]);
+  const f32x2 r2 = fma2(rz, rz, fma2(rx, rx, mul2(ry, ry)));
+  const float2 s2 = pair(r2);
+  const f32x2 ir = packed(make_float2(s2.x > rc2 ? pair_rsqrt(s2.x) : 0.0f,
+                                      second && s2.y > rc2 ? pair_rsqrt(s2.y) : 0.0f));
+  const float2 x = pair(rx), y = pair(ry), z = pair(rz);
+  if constexpr (HELM) {
+    const f32x2 kr = mul2(k, mul2(r2, ir)), ikr = mul2(ir, kinv);
+    f32x2 sn, cs;
+    sincos_near(kr, &sn, &cs);
+    // h0 = a - i b, h1 = c - i d
+    const f32x2 a = mul2(sn, ikr), b = mul2(cs, ikr);
+    const float2 q0 = reinterpret_cast<const float2*>(tl.q)[j0],
+                 q1 = reinterpret_cast<const float2*>(tl.q)[j1];
+    const f32x2 qr = packed(make_float2(q0.x, q1.x)), qi = packed(make_float2(q0.y, q1.y));
+    if (POT) {
+      const float2 a2 = pair(a), b2 = pair(b);
+      acc[0] = fmaf(a2.x, q0.x, fmaf(b2.x, q0.y, acc[0]));
+      acc[1] = fmaf(-b2.x, q0.x, fmaf(a2.x, q0.y, acc[1]));
+      acc[0] = fmaf(a2.y, q1.x, fmaf(b2.y, q1.y, acc[0]));
+      acc[1] = fmaf(-b2.y, q1.x, fmaf(a2.y, q1.y, acc[1]));
+    }
+    if (GRAD) {
+      const f32x2 c = fma2(a, ikr, mul2(b, m1)), d = fma2(b, ikr, a);
+      const float2 ar = pair(mul2(fma2(c, qr, mul2(d, qi)), ir));
+      const float2 ai = pair(mul2(fma2(c, qi, mul2(d, mul2(qr, m1))), ir));
+      acc[2] = fmaf(ar.x, x.x, acc[2]); acc[3] = fmaf(ai.x, x.x, acc[3]);
+      acc[4] = fmaf(ar.x, y.x, acc[4]); acc[5] = fmaf(ai.x, y.x, acc[5]);
+      acc[6] = fmaf(ar.x, z.x, acc[6]); acc[7] = fmaf(ai.x, z.x, acc[7]);
+      acc[2] = fmaf(ar.y, x.y, acc[2]); acc[3] = fmaf(ai.y, x.y, acc[3]);
+      acc[4] = fmaf(ar.y, y.y, acc[4]); acc[5] = fmaf(ai.y, y.y, acc[5]);
+      acc[6] = fmaf(ar.y, z.y, acc[6]); acc[7] = fmaf(ai.y, z.y, acc[7]);
+    }
+  } else {
+    const f32x2 q = packed(make_float2(tl.q[j0], tl.q[j1]));
+    if (POT) {
+      const float2 q2 = pair(q), i2 = pair(ir);
+      acc[0] = fmaf(q2.y, i2.y, fmaf(q2.x, i2.x, acc[0]));
+    }
+    if (GRAD) {
+      const float2 g = pair(mul2(q, mul2(ir, mul2(ir, ir))));
+      acc[1] = fmaf(-g.y, x.y, fmaf(-g.x, x.x, acc[1]));
+      acc[2] = fmaf(-g.y, y.y, fmaf(-g.x, y.x, acc[2]));
+      acc[3] = fmaf(-g.y, z.y, fmaf(-g.x, z.x, acc[3]));
+    }
+  }
+}
+
 // the constant factor of accumulator c of p2p_pair (see there)
 template <bool HELM>
 __device__ __forceinline__ double p2p_scale(int c, double k) {
@@ -206,17 +302,30 @@ __device__ __forceinline__ double p2p_scale(int c, double k) {
 // DIP: dipole sources (p.dip set), fixed at compile time so that the
 // monopole kernels carry no dipole code (a smaller loop body: fewer
 // instruction-fetch stalls)
-template <typename T, bool HELM, int NT, bool POT, bool GRAD, bool DIP>
+// SHARE (FP32 form): several CTAs per box.  A lane takes whole runs of terms,
+// those that a CTA with all the box's targets would sum, so that the sums do
+// not depend on the shares; its entries are then 8 apart, and the tile holds
+// entry j at tile_at(j), where lanes of neighbouring runs read neighbours
+template <int NT, bool SHARE>
+__device__ __forceinline__ int tile_at(int j) {
+  return SHARE ? (j & (kP2PRun - 1)) * (NT / kP2PRun) + j / kP2PRun : j;
+}
+
+template <typename T, bool HELM, int NT, bool POT, bool GRAD, bool DIP, bool SHARE = false>
 __global__ void __launch_bounds__(NT, NT == 32 ? 20 : (HELM ? 4 : 5))
 k_p2p(EvalParams<T> p) {
   constexpr bool F32 = sizeof(T) == 4;
   constexpr int NA = HELM ? 8 : 4;
+  constexpr bool PACK = F32 && !DIP;
   __shared__ P2PTile<T, HELM, NT> tl;
   __shared__ uint32_t s_st[27], s_pref[28];
   __shared__ double s_red[NA][NT];     // each lane's sums, for its target's group
   const int64_t b = blockIdx.x;
-  const uint32_t tc = p.tcount[b];
-  if (tc == 0) return;
+  // this CTA's share of the box's targets (gridDim.y CTAs per box)
+  const uint64_t all = p.tcount[b];
+  const uint32_t tc0 = (uint32_t)(all * blockIdx.y / gridDim.y),
+                 tc = (uint32_t)(all * (blockIdx.y + 1) / gridDim.y);
+  if (tc == tc0) return;
   const int tid = threadIdx.x;
   if (tid < 32) {
     uint32_t bi, bj, bk;
@@ -257,18 +366,30 @@ k_p2p(EvalParams<T> p) {
   // NT mod m targets, the lanes of a target consecutive; lane gl of a
   // target's g lanes takes tile entries gl, gl + g, ... (every lane busy
   // whatever the box's target count)
-  for (uint32_t t0 = 0; t0 < tc; t0 += NT) {
+  for (uint32_t t0 = tc0; t0 < tc; t0 += NT) {
     const int m = (int)min((uint32_t)NT, tc - t0);
     const int glo = NT / m, extra = NT - glo * m, split = extra * (glo + 1);
     const int ti = tid < split ? tid / (glo + 1) : extra + (tid - split) / glo;
     const int g = tid < split ? glo + 1 : glo;
     const int gl = tid < split ? tid % (glo + 1) : (tid - split) % glo;
     const uint32_t jt = p.tstart[b] + t0 + ti;
+    // gv: the lanes that a CTA with all the box's targets gives this target
+    // (FP32 form: they name its runs of terms, which are then the same
+    // whatever the shares)
+    int gv = g;
+    if constexpr (SHARE) {
+      const uint32_t t = t0 + ti, f = t / NT * NT;
+      const int mv = (int)min((uint64_t)NT, all - f);
+      gv = NT / mv + ((int)(t - f) < NT % mv ? 1 : 0);
+    }
     const double x = p.tx[jt], y = p.ty[jt], z = p.tz[jt];
     const float txh = (float)x, tyh = (float)y, tzh = (float)z;
     const float txl = (float)(x - (double)txh), tyl = (float)(y - (double)tyh),
                 tzl = (float)(z - (double)tzh);
     double a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    [[maybe_unused]] const f32x2 tt[3] = {packed(make_float2(txh, txl)),
+                                          packed(make_float2(tyh, tyl)),
+                                          packed(make_float2(tzh, tzl))};
     for (uint32_t f0 = 0; f0 < total; f0 += NT) {
       const uint32_t f = f0 + tid;
       __syncthreads();
@@ -277,30 +398,62 @@ k_p2p(EvalParams<T> p) {
         while (l < 26 && s_pref[l + 1] <= f) l++;
         const uint32_t s = s_st[l] + (f - s_pref[l]);
         const double sx = p.x[s], sy = p.y[s], sz = p.z[s];
+        const int at = tile_at<NT, SHARE>(tid);
         if constexpr (F32) {
           const float hx = (float)sx, hy = (float)sy, hz = (float)sz;
-          xp[tid] = make_float2(hx, (float)(sx - (double)hx));
-          yp[tid] = make_float2(hy, (float)(sy - (double)hy));
-          zp[tid] = make_float2(hz, (float)(sz - (double)hz));
+          xp[at] = make_float2(hx, (float)(sx - (double)hx));
+          yp[at] = make_float2(hy, (float)(sy - (double)hy));
+          zp[at] = make_float2(hz, (float)(sz - (double)hz));
         } else {
-          tl.x[tid] = sx; tl.y[tid] = sy; tl.z[tid] = sz;
+          tl.x[at] = sx; tl.y[at] = sy; tl.z[at] = sz;
         }
         if (HELM) {
-          tl.q[2 * tid] = hq ? p.q[2 * s] : T(0);
-          tl.q[2 * tid + 1] = hq ? p.q[2 * s + 1] : T(0);
-          if (hd) { tl.d[2 * tid] = p.dip[2 * s]; tl.d[2 * tid + 1] = p.dip[2 * s + 1]; }
+          tl.q[2 * at] = hq ? p.q[2 * s] : T(0);
+          tl.q[2 * at + 1] = hq ? p.q[2 * s + 1] : T(0);
+          if (hd) { tl.d[2 * at] = p.dip[2 * s]; tl.d[2 * at + 1] = p.dip[2 * s + 1]; }
         } else {
-          tl.q[tid] = hq ? p.q[s] : T(0);
-          if (hd) tl.d[tid] = p.dip[s];
+          tl.q[at] = hq ? p.q[s] : T(0);
+          if (hd) tl.d[at] = p.dip[s];
         }
-        if (hd) { tl.nx[tid] = p.nx[s]; tl.ny[tid] = p.ny[s]; tl.nz[tid] = p.nz[s]; }
+        if (hd) { tl.nx[at] = p.nx[s]; tl.ny[at] = p.ny[s]; tl.nz[at] = p.nz[s]; }
       }
       __syncthreads();
       const int nt = (int)min((uint32_t)NT, total - f0);
-      if constexpr (F32) {
+      if constexpr (PACK) {
+        // runs of kP2PRun pairs, two at a time: a full run without bounds
+        // checks, the tile's last run with them
+        const f32x2 kk = both(k), ki = both(kinv);
+        auto two = [&](int j0, int j1, bool second, float* acc) {
+          p2p_two<HELM, NT, POT, GRAD>(tl, tile_at<NT, SHARE>(j0), tile_at<NT, SHARE>(j1), second,
+                                       tt, rc2, kk, ki, acc);
+        };
+        for (int w = gl;; w += g) {
+          const int j0 = SHARE ? w % gv + w / gv * (kP2PRun * gv) : gl + (w - gl) * kP2PRun;
+          if (j0 >= nt) {
+            if (!SHARE || w / gv * (kP2PRun * gv) >= nt) break;
+            continue;
+          }
+          float acc[NA];
+#pragma unroll
+          for (int c = 0; c < NA; c++) acc[c] = 0.0f;
+          if (j0 + (kP2PRun - 1) * gv < nt) {
+#pragma unroll
+            for (int u = 0; u < kP2PRun; u += 2) two(j0 + u * gv, j0 + (u + 1) * gv, true, acc);
+          } else {
+#pragma unroll 1
+            for (int u = 0; u < kP2PRun && j0 + u * gv < nt; u += 2) {
+              const int j = j0 + u * gv;
+              two(j, j + gv < nt ? j + gv : j, j + gv < nt, acc);
+            }
+          }
+#pragma unroll
+          for (int c = 0; c < NA; c++) a[c] += (double)acc[c];
+        }
+      } else if constexpr (F32) {
         // runs of kP2PRun pairs: a full run without bounds checks, the
         // tile's last run with them; the cutoff by masking (p2p_pair)
-        auto pair_at = [&](int j, T* acc) {
+        auto pair_at = [&](int entry, T* acc) {
+          const int j = tile_at<NT, SHARE>(entry);
           const float2 cx = xp[j], cy = yp[j], cz = zp[j];
           const T rx = (T)((txh - cx.x) + (txl - cx.y));
           const T ry = (T)((tyh - cy.x) + (tyl - cy.y));
@@ -308,16 +461,21 @@ k_p2p(EvalParams<T> p) {
           const T r2 = rx * rx + ry * ry + rz * rz;
           p2p_pair<T, HELM, NT, POT, GRAD, true>(tl, j, rx, ry, rz, r2, k, kinv, hd, acc, rc2);
         };
-        for (int j0 = gl; j0 < nt; j0 += kP2PRun * g) {
+        for (int w = gl;; w += g) {
+          const int j0 = SHARE ? w % gv + w / gv * (kP2PRun * gv) : gl + (w - gl) * kP2PRun;
+          if (j0 >= nt) {
+            if (!SHARE || w / gv * (kP2PRun * gv) >= nt) break;
+            continue;
+          }
           T acc[NA];
           for (int c = 0; c < NA; c++) acc[c] = T(0);
-          if (j0 + (kP2PRun - 1) * g < nt) {
+          if (j0 + (kP2PRun - 1) * gv < nt) {
 #pragma unroll
-            for (int u = 0; u < kP2PRun; u++) pair_at(j0 + u * g, acc);
+            for (int u = 0; u < kP2PRun; u++) pair_at(j0 + u * gv, acc);
           } else {
 #pragma unroll
             for (int u = 0; u < kP2PRun; u++)
-              if (j0 + u * g < nt) pair_at(j0 + u * g, acc);
+              if (j0 + u * gv < nt) pair_at(j0 + u * gv, acc);
           }
           for (int c = 0; c < NA; c++) a[c] += (double)acc[c];
         }
@@ -366,10 +524,22 @@ int launch_p2p(const EvalParams<T>& p, cudaStream_t s) {
   auto go = [&](auto pot, auto grad, auto dip) {
     constexpr bool P = decltype(pot)::value, G = decltype(grad)::value;
     constexpr bool D = decltype(dip)::value;
+    // a tree with fewer leaves than two per SM (depth 2 at most): several
+    // CTAs share a box's targets, in shares of 64, 32, 16 or 8 on average,
+    // the largest that give four CTAs per SM (1e4 FP32 Laplace points in 64
+    // leaves: 218 us with a CTA per leaf, on 64 of 148 SMs)
+    int64_t y = 1;
+    if (p.nbox < 2 * 148)
+      for (int64_t share = 64; share >= 8 && p.nbox * y < 4 * 148; share /= 2)
+        y = (p.ntgt + p.nbox * share - 1) / (p.nbox * share);
+    if (y > 65535) y = 65535;
+    const dim3 grid((unsigned)p.nbox, (unsigned)(y < 1 ? 1 : y));
     if (p.ntgt <= 8 * p.nbox)   // a few targets per leaf on average
-      k_p2p<T, HELM, 32, P, G, D><<<(unsigned)p.nbox, 32, 0, s>>>(p);
+      k_p2p<T, HELM, 32, P, G, D><<<grid, 32, 0, s>>>(p);   // (y is 1)
+    else if (sizeof(T) == 4 && grid.y > 1)
+      k_p2p<T, HELM, 128, P, G, D, sizeof(T) == 4><<<grid, 128, 0, s>>>(p);
     else
-      k_p2p<T, HELM, 128, P, G, D><<<(unsigned)p.nbox, 128, 0, s>>>(p);
+      k_p2p<T, HELM, 128, P, G, D><<<grid, 128, 0, s>>>(p);
   };
   auto fields = [&](auto dip) {
     if (p.pot && p.grad) go(std::true_type(), std::true_type(), dip);
@@ -413,10 +583,15 @@ __global__ void k_sincos_check(double xmax, int n, double* err) {
   for (int i = threadIdx.x; i <= n; i += blockDim.x) {
     const float x = (float)(xmax * i / n);
     float s, c, s1, c1;
-    sincos_near(x, &s, &c);
+    f32x2 sp, cp;
+    sincos_near(both(x), &sp, &cp);
+    float s0, c0;
+    sincos_near(x, &s0, &c0);
+    s = pair(sp).x; c = pair(cp).y;
     sincosf(x, &s1, &c1);
     const double sd = sin((double)x), cd = cos((double)x);
     e0 = fmax(e0, fmax(fabs(s - sd), fabs(c - cd)));
+    e0 = fmax(e0, fmax(fabs(s0 - sd), fabs(c0 - cd)));
     e1 = fmax(e1, fmax(fabs(s1 - sd), fabs(c1 - cd)));
   }
   m[0][threadIdx.x] = e0; m[1][threadIdx.x] = e1;
