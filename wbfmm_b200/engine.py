@@ -279,8 +279,8 @@ class Solver:
         _check(self.lib.wbfmm_b200_downward_pass(self.h, level))
 
     def set_m2l_kernel(self, mode):
-        """0 warp per target, 1 automatic (default), 2 lane per pair, 3 target
-        tiles; True / False select 1 / 0."""
+        """0 warp per target, 1 automatic (default), 2 lane per pair, 3 columns
+        or target tiles; True / False select 1 / 0."""
         _check(self.lib.wbfmm_b200_set_m2l_kernel(self.h, int(mode)))
 
     def m2l(self, level):
