@@ -527,7 +527,7 @@ int launch_p2p(const EvalParams<T>& p, cudaStream_t s) {
     // a tree with fewer leaves than two per SM (depth 2 at most): several
     // CTAs share a box's targets, in shares of 64, 32, 16 or 8 on average,
     // the largest that give four CTAs per SM (1e4 FP32 Laplace points in 64
-    // leaves: 218 us with a CTA per leaf, on 64 of 148 SMs)
+    // leaves: 218 us with a CTA per leaf, on 64 of 148 SMs, about 125 so)
     int64_t y = 1;
     if (p.nbox < 2 * 148)
       for (int64_t share = 64; share >= 8 && p.nbox * y < 4 * 148; share /= 2)
