@@ -1,6 +1,7 @@
 """P2M with a few points per leaf (8 lanes per box) against a warp per box: the
-rule changes sides at 12 points per leaf on average, so a problem on it and the
-same problem with one more source of strength zero take the two forms."""
+rule changes sides at 12 points per leaf on average (from 24 leaves per SM), so
+a problem on it and the same problem with one more source of strength zero take
+the two forms."""
 from __future__ import annotations
 
 import numpy as np
@@ -19,7 +20,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("dipoles", [False, True])
 def test_p2m_forms(gpu_lib, problem, precision, tol, order, dipoles):
     rng = np.random.default_rng(order)
-    depth, n = 2, 12 * 64
+    depth, n = 4, 12 * 4096
     w = 2 if problem == engine.HELMHOLTZ else 1
     pts = rng.uniform(-0.5, 0.5, (n, 3))
     pts[:40] = rng.uniform(0.3, 0.31, (40, 3))          # one leaf with more points than lanes
@@ -27,7 +28,7 @@ def test_p2m_forms(gpu_lib, problem, precision, tol, order, dipoles):
     nrm = rng.standard_normal((n, 3))
     nrm /= np.linalg.norm(nrm, axis=1, keepdims=True)
     orders = [0] + [order] * depth
-    cfg = engine.SolverConfig(problem, depth, orders, list(orders), 6.0, (-0.51,) * 3, 1.02, precision)
+    cfg = engine.SolverConfig(problem, depth, orders, list(orders), 16.0, (-0.51,) * 3, 1.02, precision)
 
     def leaves(extra):
         z = np.zeros((extra, w))

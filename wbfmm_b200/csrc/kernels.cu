@@ -165,46 +165,65 @@ __global__ void k_p2m(P2MParams<T> p, int legt, int share) {
     if (most > 0) {
       for (int c = gl; c < nc * w; c += G) acc[c] = T(0);
       __syncwarp();
-      double cd[3];
-      box_centre(b, p.x0, p.y0, p.z0, p.wb, cd);
-      // source position relative to the box centre, formed in FP64
-      const T xc[3] = {T(0), T(0), T(0)};
-      for (uint32_t base = share ? warp * G : 0; base < most; base += share ? nw * G : G) {
-        const uint32_t t = base + gl;
-        const bool act = t < cnt;
-        const uint32_t s = act ? start + t : 0;
-        T xs[3] = {act ? (T)(p.x[s] - cd[0]) : T(0),
-                   act ? (T)(p.y[s] - cd[1]) : T(0),
-                   act ? (T)(p.z[s] - cd[2]) : T(0)};
-        auto expand = [&](const auto& leg) {
-          if (HELM) {
-            const P2MEmitHelm<T, G> emit{acc, lane};
-            if (p.q) {
-              T qr = act ? p.q[2 * s] : T(0), qi = act ? p.q[2 * s + 1] : T(0);
-              p2m_helmholtz<T>(N, p.k, xc, xs, qr, qi, emit, leg, sc);
+      // the points of box b, W lanes at a time
+      auto points = [&](auto lanes, int64_t b, uint32_t cnt, uint32_t start, uint32_t most, T* acc) {
+        constexpr int W = decltype(lanes)::value;
+        double cd[3];
+        box_centre(b, p.x0, p.y0, p.z0, p.wb, cd);
+        // source position relative to the box centre, formed in FP64
+        const T xc[3] = {T(0), T(0), T(0)};
+        for (uint32_t base = share ? warp * W : 0; base < most; base += share ? nw * W : W) {
+          const uint32_t t = base + (lane & (W - 1));
+          const bool act = t < cnt;
+          const uint32_t s = act ? start + t : 0;
+          T xs[3] = {act ? (T)(p.x[s] - cd[0]) : T(0),
+                     act ? (T)(p.y[s] - cd[1]) : T(0),
+                     act ? (T)(p.z[s] - cd[2]) : T(0)};
+          auto expand = [&](const auto& leg) {
+            if (HELM) {
+              const P2MEmitHelm<T, W> emit{acc, lane};
+              if (p.q) {
+                T qr = act ? p.q[2 * s] : T(0), qi = act ? p.q[2 * s + 1] : T(0);
+                p2m_helmholtz<T>(N, p.k, xc, xs, qr, qi, emit, leg, sc);
+              }
+              if (p.dip) {
+                T dr = act ? p.dip[2 * s] : T(0), di = act ? p.dip[2 * s + 1] : T(0);
+                T nrm[3] = {act ? p.nx[s] : T(0), act ? p.ny[s] : T(0),
+                            act ? p.nz[s] : T(1)};
+                p2m_helmholtz_dipole<T>(N, p.k, xc, xs, nrm, dr, di, emit, leg, sc);
+              }
+            } else {
+              const P2MEmitLap<T, W> emit{acc, lane};
+              if (p.q) {
+                T qv = act ? p.q[s] : T(0);
+                p2m_laplace<T>(N, xc, xs, qv, emit, leg, sc);
+              }
+              if (p.dip) {
+                T dv = act ? p.dip[s] : T(0);
+                T nrm[3] = {act ? p.nx[s] : T(0), act ? p.ny[s] : T(0),
+                            act ? p.nz[s] : T(1)};
+                p2m_laplace_dipole<T>(N, xc, xs, nrm, dv, emit, leg, sc);
+              }
             }
-            if (p.dip) {
-              T dr = act ? p.dip[2 * s] : T(0), di = act ? p.dip[2 * s + 1] : T(0);
-              T nrm[3] = {act ? p.nx[s] : T(0), act ? p.ny[s] : T(0),
-                          act ? p.nz[s] : T(1)};
-              p2m_helmholtz_dipole<T>(N, p.k, xc, xs, nrm, dr, di, emit, leg, sc);
-            }
-          } else {
-            const P2MEmitLap<T, G> emit{acc, lane};
-            if (p.q) {
-              T qv = act ? p.q[s] : T(0);
-              p2m_laplace<T>(N, xc, xs, qv, emit, leg, sc);
-            }
-            if (p.dip) {
-              T dv = act ? p.dip[s] : T(0);
-              T nrm[3] = {act ? p.nx[s] : T(0), act ? p.ny[s] : T(0),
-                          act ? p.nz[s] : T(1)};
-              p2m_laplace_dipole<T>(N, xc, xs, nrm, dv, emit, leg, sc);
-            }
-          }
-        };
-        if (legt) expand(LegTab<T>{lt, LW});
-        else expand(LegDirect<T>());
+          };
+          if (legt) expand(LegTab<T>{lt, LW});
+          else expand(LegDirect<T>());
+        }
+      };
+      // boxes of very unequal counts one after the other, a warp each, where
+      // that takes fewer rounds
+      if (NG > 1 && __reduce_add_sync(0xffffffffu, gl == 0 ? (cnt + 31) / 32 : 0) <
+                        (most + G - 1) / G) {
+#pragma unroll 1
+        for (int i = 0; i < NG; i++) {
+          const uint32_t ci = __shfl_sync(0xffffffffu, cnt, i * G);
+          const uint32_t si = __shfl_sync(0xffffffffu, start, i * G);
+          const int64_t bi = __shfl_sync(0xffffffffu, (long long)b, i * G);
+          points(std::integral_constant<int, 32>(), bi, ci, si, ci,
+                 acc + (size_t)(i - lane / G) * nc * w);
+        }
+      } else {
+        points(std::integral_constant<int, G>(), b, cnt, start, most, acc);
       }
       __syncwarp();
     }
@@ -242,11 +261,14 @@ int launch_p2m(const P2MParams<T>& p, cudaStream_t s) {
   const size_t leg = leg_table_bytes<T>(p.N);
   const size_t rows = p2m_row_bytes<T>(p.N, nw * 32);
   const size_t one = sizeof(T) * (size_t)nw * ncoef(p.N) * (HELM ? 2 : 1);   // a box per warp
-  // leaves of up to 12 points on average: four boxes per warp, while their
+  // leaves of up to 12 points on average: four boxes per warp (in turn where
+  // their counts differ much: clustered points, 2375 in 512 leaves, Laplace
+  // order 15 with dipoles, took 3.1 ms against 1.9 without that), while their
   // accumulators leave room for a second CTA; not where most boxes are empty
   // and the others full (surface points, 33 per occupied leaf: 4.2 ms against
-  // 3.1)
-  const bool few = !p.skewed && p.npts <= 12 * p.nbox && leg + rows + 4 * one <= 100 * 1024;
+  // 3.1), and not below 24 boxes per SM, which a warp each does not fill: there
+  // the longest warp counts (8^3 boxes of clustered points: 2.2 ms against 1.9)
+  const bool few = !p.skewed && p.nbox >= 148 * 24 && p.npts <= 12 * p.nbox && leg + rows + 4 * one <= 100 * 1024;
   const bool share = !few && p.nbox <= 148 * 8 && p.npts > 48 * p.nbox;
   auto go = [&](auto srows, auto nc, auto group) -> int {
     constexpr bool SR = decltype(srows)::value;
