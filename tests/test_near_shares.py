@@ -71,3 +71,31 @@ def test_near(gpu_lib, problem, precision, tol, ns, nt, dipoles):
         got_p, got_g = got_p[0::2] + 1j * got_p[1::2], got_g[0::2] + 1j * got_g[1::2]
     assert np.linalg.norm(got_p - P) <= tol * np.linalg.norm(P)
     assert np.linalg.norm(got_g - G.ravel()) <= tol * np.linalg.norm(G)
+
+
+# An infinite strength reaches every target of its leaf as an infinity and not
+# as a NaN, whichever entry of a run it is (lone ones among them), as in the
+# kernel for dipole sources (here of strength zero), whose terms are not paired
+@pytest.mark.parametrize("problem", [engine.LAPLACE, engine.HELMHOLTZ])
+@pytest.mark.parametrize("ns,nt,depth", [(1, 1, 2), (7, 40, 2), (5, 600, 2), (7, 5000, 3)])
+def test_infinite_strength(gpu_lib, problem, ns, nt, depth):
+    rng = np.random.default_rng(ns + nt)
+    w = 2 if problem == engine.HELMHOLTZ else 1
+    xs, xt = rng.uniform(0.01, 0.11, (ns, 3)), rng.uniform(0.01, 0.11, (nt, 3))
+    nrm = np.tile([0.0, 0.0, 1.0], (ns, 1))
+    orders = [0] + [6] * depth
+    cfg = engine.SolverConfig(problem, depth, orders, list(orders), 6.0, (-0.51,) * 3, 1.02,
+                              engine.FP32, engine.POTENTIAL | engine.GRADIENT)
+    zero = np.zeros(ns * w)
+    with engine.Solver(cfg) as s:
+        s.set_sources(xs, nrm).set_strengths(zero).set_targets(xt).run()   # no far field
+        for i in range(ns):
+            q = rng.uniform(0.5, 1.0, ns * w)
+            q[i * w] = np.inf
+            fields = []
+            for dip in (None, zero):
+                s.set_strengths(q, dip)
+                s.evaluate()
+                fields.append(np.concatenate([np.ravel(f) for f in s.field()]))
+            assert np.all(np.isinf(fields[1]))
+            assert np.array_equal(fields[0], fields[1])

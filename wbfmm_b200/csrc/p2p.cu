@@ -226,7 +226,8 @@ __device__ __forceinline__ void sincos_near(f32x2 x, f32x2* sp, f32x2* cp) {
 // p2p_pair (monopoles, cutoff masked) of tile entries j0 and j1, the terms
 // two at a time in packed arithmetic (f32x2.cuh) and then added one after
 // the other: the operations and the order of sums of two calls of p2p_pair.
-// second: false for a lone entry j0 (1/r of the other is then 0).
+// second: false for a lone entry j0, whose partner counts nothing: 1/r and
+// strength zero (1/r alone would not do: 0 x Inf of an infinite strength).
 // t: the target's coordinates, each hi and lo
 template <bool HELM, int NT, bool POT, bool GRAD>
 __device__ __forceinline__ void p2p_two(const P2PTile<float, HELM, NT>& tl, int j0, int j1,
@@ -251,7 +252,7 @@ __device__ __forceinline__ void p2p_two(const P2PTile<float, HELM, NT>& tl, int 
     // h0 = a - i b, h1 = c - i d
     const f32x2 a = mul2(sn, ikr), b = mul2(cs, ikr);
     const float2 q0 = reinterpret_cast<const float2*>(tl.q)[j0],
-                 q1 = reinterpret_cast<const float2*>(tl.q)[j1];
+                 q1 = second ? reinterpret_cast<const float2*>(tl.q)[j1] : make_float2(0.0f, 0.0f);
     const f32x2 qr = packed(make_float2(q0.x, q1.x)), qi = packed(make_float2(q0.y, q1.y));
     if (POT) {
       const float2 a2 = pair(a), b2 = pair(b);
@@ -272,7 +273,7 @@ __device__ __forceinline__ void p2p_two(const P2PTile<float, HELM, NT>& tl, int 
       acc[6] = fmaf(ar.y, z.y, acc[6]); acc[7] = fmaf(ai.y, z.y, acc[7]);
     }
   } else {
-    const f32x2 q = packed(make_float2(tl.q[j0], tl.q[j1]));
+    const f32x2 q = packed(make_float2(tl.q[j0], second ? tl.q[j1] : 0.0f));
     if (POT) {
       const float2 q2 = pair(q), i2 = pair(ir);
       acc[0] = fmaf(q2.y, i2.y, fmaf(q2.x, i2.x, acc[0]));
