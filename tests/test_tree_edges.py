@@ -33,3 +33,25 @@ def test_tree(restatement, gpu_lib, n, kind):
             assert np.array_equal(ip, want)
             sl = slice(off[lv], off[lv] + 8 ** lv)
             assert np.array_equal(bi, boxes[sl, 0]) and np.array_equal(bn, boxes[sl, 1])
+
+
+# a refused set_sources (a point on the cube's face) leaves the sources in
+# place: new strengths give the fields they gave before
+@pytest.mark.parametrize("n", [3000, 6000])            # both sorts
+@pytest.mark.parametrize("refused", ["same", "fewer", "more"])
+def test_refused_sources_keep_the_tree(gpu_lib, n, refused):
+    rng = np.random.default_rng(n)
+    pts, q = rng.uniform(-0.5, 0.5, (n, 3)), rng.standard_normal(n)
+    bad = rng.uniform(-0.5, 0.5, ({"same": n, "fewer": n // 2, "more": 2 * n}[refused], 3))
+    bad[7, 1] = -0.51
+    cfg = engine.SolverConfig(engine.LAPLACE, 3, [0, 6, 6, 6], [0, 6, 6, 6], 0.0, (-0.51,) * 3, 1.02,
+                              engine.FP64, engine.POTENTIAL | engine.GRADIENT)
+    with engine.Solver(cfg) as s:
+        want = s.set_sources(pts).set_strengths(q).set_targets(pts).run().field()
+        with pytest.raises(engine.WbfmmError):
+            s.set_sources(bad)
+        got = s.set_strengths(q).run().field()
+        for a, b in zip(got, want):
+            assert np.array_equal(a, b)
+        ip, _, bn = s.tree(3)
+        assert np.array_equal(np.sort(ip), np.arange(n)) and bn.sum() == n

@@ -62,8 +62,8 @@ int ensure_smem(size_t bytes) {
 // *a = va and, when b is non-null, *b = vb (one thread, on stream s)
 void launch_set_words(uint32_t* a, uint32_t va, uint32_t* b, uint32_t vb,
                       cudaStream_t s);
-// keys[i] = Morton key of point i (src/boxes.c:324-339); vals[i] = i; with
-// bad non-null the strict-interior domain check of the sources
+// keys[i] = Morton key of point i (src/boxes.c:324-339); vals[i] = i (neither
+// where keys is null); with bad non-null the strict-interior domain check of the sources
 // (src/boxes.c:148-153): *bad = min(*bad, first point outside).
 // f32: in FP32 arithmetic, as the single-precision build (the *_f API), on
 // coordinates, origin and width that are FP32 values

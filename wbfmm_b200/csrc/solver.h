@@ -428,8 +428,6 @@ struct Solver : public wbfmm_b200_solver {
     gen++;
     geo++;
     src_arg = nullptr;              // set again only when these sources are in place
-    nsrc = n;
-    xstr = xs_str;
     const double* dpts = xs;
     if (!on_device) {
       WBFMM_TRY(pts_in.alloc((size_t)n * xs_str));
@@ -437,18 +435,25 @@ struct Solver : public wbfmm_b200_solver {
                                  cudaMemcpyHostToDevice, stream));
       dpts = pts_in.p;
     }
-    // strict-interior domain check (src/boxes.c:148-153)
+    // strict-interior domain check (src/boxes.c:148-153): with the keys where
+    // it is read back after the solve, else before anything of the sources in
+    // place is overwritten (a caller may go on with them after a refusal)
     launch_set_words((uint32_t*)flag.p, 0x7fffffffu, (uint32_t*)flag.p + 2, 0, stream);
-    WBFMM_TRY(keys.alloc(n));
-    WBFMM_TRY(ip.alloc(n));
-    launch_point_keys(dpts, xs_str, n, cfg.x0, cfg.D, keys.p, ip.p, flag.p, stream,
-                      cfg.keys_fp32 != 0);
     if (!async_checks) {
+      launch_point_keys(dpts, xs_str, n, cfg.x0, cfg.D, nullptr, nullptr, flag.p, stream,
+                        cfg.keys_fp32 != 0);
       int bad = 0;
       WBFMM_CUDA(cudaMemcpyAsync(&bad, flag.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
       WBFMM_CUDA(cudaStreamSynchronize(stream));
       WBFMM_TRY(domain_error(bad, 0));
+      launches++;
     }
+    nsrc = n;
+    xstr = xs_str;
+    WBFMM_TRY(keys.alloc(n));
+    WBFMM_TRY(ip.alloc(n));
+    launch_point_keys(dpts, xs_str, n, cfg.x0, cfg.D, keys.p, ip.p,
+                      async_checks ? flag.p : nullptr, stream, cfg.keys_fp32 != 0);
     // full 60-bit keys (the reference's point order), or with leaf_order
     // only the bits that select the leaf box
     const int sort_lo = cfg.leaf_order ? 60 - 3 * depth : 0;

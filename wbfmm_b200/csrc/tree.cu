@@ -111,8 +111,8 @@ __device__ __forceinline__ bool outside_open(double x, double x0, double D, bool
   return x <= x0 || x >= x0 + D;
 }
 
-// the key of every point, and with `bad` the strict-interior check: *bad the
-// first point outside
+// the key of every point (unless keys is null), and with `bad` the
+// strict-interior check: *bad the first point outside
 __global__ void k_point_keys(const double* __restrict__ pts, int64_t pstr,
                              int n, double x0, double y0, double z0, double D,
                              uint64_t* __restrict__ keys,
@@ -124,6 +124,7 @@ __global__ void k_point_keys(const double* __restrict__ pts, int64_t pstr,
   if (bad && (outside_open(x, x0, D, f32) || outside_open(y, y0, D, f32) ||
               outside_open(z, z0, D, f32)))
     atomicMin(bad, i);
+  if (!keys) return;
   uint32_t xi = key_coord(x, x0, D, f32);
   uint32_t yi = key_coord(y, y0, D, f32);
   uint32_t zi = key_coord(z, z0, D, f32);
