@@ -4,6 +4,10 @@ or 8 and 16 per warp tile, the column counts of its shared-memory plans), on
 dense levels, target lists and sparse storage."""
 from __future__ import annotations
 
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -66,3 +70,45 @@ def test_target_lists_and_sparse(problem, precision, tol, order):
         _, (f, g) = _locals(p, precision, 3, **kw)
         assert np.linalg.norm(f - pot) < tol * np.linalg.norm(pot)
         assert np.linalg.norm(g - grad) < tol * np.linalg.norm(grad)
+
+
+FIRST_USE = r"""
+import threading
+import numpy as np
+from wbfmm_b200 import engine, workloads as W
+
+def solve(problem, order, out, i, start=None):
+    p = W.serve_request(np.random.default_rng(order), 2003, problem == engine.HELMHOLTZ, 18.0, False)
+    p.depth, p.order_s = 3, [0] + [order] * 3
+    p.order_r = list(p.order_s)
+    with engine.Solver(engine.SolverConfig.from_problem(p, engine.FP64)) as s:
+        s.set_sources(p.xs).set_strengths(p.q).set_targets(p.xt)
+        s.build_operators()
+        s.synchronize()
+        if start is not None:
+            start.wait()
+        out[i] = s.run().field()
+
+# lanes, columns, and (FP64 Laplace, level 2) tiles
+cases = [(engine.LAPLACE, 7), (engine.HELMHOLTZ, 8), (engine.LAPLACE, 12)] * 3
+first, again = [None] * len(cases), [None] * len(cases)
+start = threading.Barrier(len(cases))
+threads = [threading.Thread(target=solve, args=(*c, first, i, start)) for i, c in enumerate(cases)]
+for t in threads:
+    t.start()
+for t in threads:
+    t.join()
+for i, c in enumerate(cases):
+    solve(*c, again, i)
+for a, b in zip(first, again):
+    assert all(np.array_equal(x, y) for x, y in zip(a, b))
+print("same")
+"""
+
+
+def test_first_use_by_several_threads(gpu_lib):
+    """The first M2L launches of a process, from several threads on streams of
+    their own: each waits for its kernel's table of offsets."""
+    r = subprocess.run([sys.executable, "-c", FIRST_USE], capture_output=True, text=True, timeout=300,
+                       cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0 and "same" in r.stdout, r.stderr[-2000:]

@@ -59,6 +59,29 @@ int ensure_smem(size_t bytes) {
   } while (0)
 
 // ------------------------------------------------------------------ tree
+// What is done once per device before its first use there, such as filling a
+// constant table: `upload` under a lock, then a wait for the default stream,
+// on which cudaMemcpyToSymbol copies (a copy from pageable memory may return
+// before it has arrived, and kernels of non-blocking streams are not ordered
+// after it).
+class DeviceOnce {
+  std::mutex mu;
+  bool done[64] = {false};
+
+ public:
+  template <class F>
+  int run(F&& upload) {
+    int dev = 0;
+    WBFMM_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(mu);
+    if (dev < 64 && done[dev]) return 0;
+    if (const int rc = upload()) return rc;
+    WBFMM_CUDA(cudaStreamSynchronize(0));
+    if (dev < 64) done[dev] = true;
+    return 0;
+  }
+};
+
 // *a = va and, when b is non-null, *b = vb (one thread, on stream s)
 void launch_set_words(uint32_t* a, uint32_t va, uint32_t* b, uint32_t vb,
                       cudaStream_t s);

@@ -52,7 +52,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <mutex>
 
 #include "engine.h"
 #include "f32x2.cuh"
@@ -234,30 +233,26 @@ int cols_ctas(size_t smem) { return 2 * (smem + 1024) <= 228 * 1024 ? 2 : 1; }
 // per target type: the 189 offsets ordered by rotation angle, then distance:
 // the packed code of build_offset_table | distance index << 18 | angle << 22
 __constant__ int c_cols_offsets[8][189];
-std::mutex g_cols_mu;
-bool g_cols_ready[64] = {false};
+DeviceOnce g_cols_offsets;
 
 int ensure_cols_offsets() {
-  int dev = 0;
-  WBFMM_CUDA(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lk(g_cols_mu);
-  if (dev < 64 && g_cols_ready[dev]) return 0;
-  int tab[8 * 189];
-  build_offset_table(tab);
-  ShiftGeometry g;
-  build_shift_geometry(&g);
-  for (int tau = 0; tau < 8; tau++) {
-    int* o = tab + tau * 189;
-    for (int j = 0; j < 189; j++) {
-      const ShiftAngles& a = g.offset[o[j] & 511];
-      o[j] |= list_dist_index(a.idist) << 18 | a.ith << 22;
+  return g_cols_offsets.run([] {
+    int tab[8 * 189];
+    build_offset_table(tab);
+    ShiftGeometry g;
+    build_shift_geometry(&g);
+    for (int tau = 0; tau < 8; tau++) {
+      int* o = tab + tau * 189;
+      for (int j = 0; j < 189; j++) {
+        const ShiftAngles& a = g.offset[o[j] & 511];
+        o[j] |= list_dist_index(a.idist) << 18 | a.ith << 22;
+      }
+      std::stable_sort(o, o + 189, [](int a, int b) { return (a >> 18) < (b >> 18); });
+      std::stable_sort(o, o + 189, [](int a, int b) { return (a >> 22) < (b >> 22); });
     }
-    std::stable_sort(o, o + 189, [](int a, int b) { return (a >> 18) < (b >> 18); });
-    std::stable_sort(o, o + 189, [](int a, int b) { return (a >> 22) < (b >> 22); });
-  }
-  WBFMM_CUDA(cudaMemcpyToSymbol(c_cols_offsets, tab, sizeof(tab)));
-  if (dev < 64) g_cols_ready[dev] = true;
-  return 0;
+    WBFMM_CUDA(cudaMemcpyToSymbol(c_cols_offsets, tab, sizeof(tab)));
+    return 0;
+  });
 }
 
 __constant__ int c_cols_dist2[15] = {4, 5, 6, 8, 9, 10, 11, 12, 13, 14, 17, 18, 19, 22, 27};

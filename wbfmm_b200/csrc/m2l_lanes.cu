@@ -41,17 +41,15 @@ template <> struct V2t<double> { typedef double2 t; };
 // per target type: 189 packed offsets (op | sigma << 9 | (dx+1) << 12 |
 // (dy+1) << 14 | (dz+1) << 16), dx.. = parent offset of the source
 __constant__ int c_offsets[8][189];
-static bool g_offsets_ready[64] = {false};
+static DeviceOnce g_offsets;
 
 static int ensure_offsets() {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 64 && g_offsets_ready[dev]) return 0;
-  int tab[8 * 189];
-  build_offset_table(tab);
-  WBFMM_CUDA(cudaMemcpyToSymbol(c_offsets, tab, sizeof(tab)));
-  if (dev < 64) g_offsets_ready[dev] = true;
-  return 0;
+  return g_offsets.run([] {
+    int tab[8 * 189];
+    build_offset_table(tab);
+    WBFMM_CUDA(cudaMemcpyToSymbol(c_offsets, tab, sizeof(tab)));
+    return 0;
+  });
 }
 
 // ----------------------------------------------------------- transpose

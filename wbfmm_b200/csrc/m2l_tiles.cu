@@ -74,17 +74,15 @@ __global__ void k_helm_coax_rows(const T* __restrict__ raw, int64_t raw_stride, 
 }
 
 __constant__ int c_tile_offsets[8][189];
-bool g_tile_offsets_ready[64] = {false};
+DeviceOnce g_tile_offsets;
 
 int ensure_tile_offsets() {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 64 && g_tile_offsets_ready[dev]) return 0;
-  int tab[8 * 189];
-  build_offset_table(tab);
-  WBFMM_CUDA(cudaMemcpyToSymbol(c_tile_offsets, tab, sizeof(tab)));
-  if (dev < 64) g_tile_offsets_ready[dev] = true;
-  return 0;
+  return g_tile_offsets.run([] {
+    int tab[8 * 189];
+    build_offset_table(tab);
+    WBFMM_CUDA(cudaMemcpyToSymbol(c_tile_offsets, tab, sizeof(tab)));
+    return 0;
+  });
 }
 
 constexpr int kTileThreads = 256;
