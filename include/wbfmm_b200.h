@@ -286,14 +286,18 @@ int wbfmm_b200_tree_structure_f(int n, const float *pts, int pstr,
    order 6 (Helmholtz) / 8 (Laplace), matrix products on columns of target
    boxes above (FP64 on the tensor cores; to order 24 in FP32, 17 / 18 in
    FP64), offset-major target tiles beyond, while their shared memory
-   suffices; 2 = lane-per-pair wherever instantiated
-   (Helmholtz <= 8, Laplace <= 10), columns elsewhere; 3 = columns, or target tiles, wherever
-   they fit;
+   suffices (and at level 2 of a dense FP64 Laplace solve from order 10 on);
+   2 = lane-per-pair wherever instantiated (Helmholtz <= 8, Laplace <= 10),
+   columns elsewhere; 3 = target tiles wherever they fit; 5 = columns wherever
+   they fit, else target tiles;
    0 = always the warp-per-target kernel; 4 = Laplace FP32 on the tensor
    cores (dense per-shift operators, tcgen05 kind::tf32 with 3xTF32
    splitting, FP32 accumulation in tensor memory) for equal orders with
    (p+1)^2 <= 256, the automatic choice elsewhere. */
 int wbfmm_b200_set_m2l_kernel(wbfmm_b200_solver_t *s, int mode);
+/* The kernel that a level's last M2L ran in: 0, 2, 3, 4 or 5 as above; -1:
+   none yet (for tests of one kernel). */
+int wbfmm_b200_selftest_m2l_form(wbfmm_b200_solver_t *s, int level);
 
 /* FP64 direct sum with self-exclusion (r <= 1e-6) and compensated
    accumulation: the GPU counterpart of wbfmm_total_field[_grad]

@@ -1,6 +1,7 @@
-"""The column M2L kernel against the warp-per-target kernel: local expansions
-at the orders where its tiles change shape (one and two row tiles, 1 to 4 rows
-or 8 and 16 per warp tile, the column counts of its shared-memory plans), on
+"""The column M2L kernel (mode 5) against the warp-per-target kernel: local
+expansions at the orders where its tiles change shape (one and two row tiles,
+1 to 4 rows or 8 and 16 per warp tile, the column counts of its shared-memory
+plans; level 2 takes one column per lane, level 3 the plan of its order), on
 dense levels, target lists and sparse storage."""
 from __future__ import annotations
 
@@ -31,6 +32,7 @@ def _locals(p, precision, mode, **kw):
     with engine.Solver(cfg) as s:
         s.set_m2l_kernel(mode)
         s.set_sources(p.xs).set_strengths(p.q).set_targets(p.xt).run()
+        assert all(s.m2l_form(lv) == mode for lv in range(2, p.depth + 1))
         return [s.coefficients(lv)[1] for lv in range(2, p.depth + 1)], s.field()
 
 
@@ -43,18 +45,20 @@ def _locals(p, precision, mode, **kw):
 def test_orders(problem, precision, tol, order):
     p = _problem(problem, order, 3, 3001, False, 18.0)
     want, _ = _locals(p, precision, 0)
-    got, _ = _locals(p, precision, 3)
+    got, _ = _locals(p, precision, 5)
     for a, b in zip(got, want):
         assert np.linalg.norm(a - b) < tol * np.linalg.norm(b)
 
 
 @pytest.mark.parametrize("problem,precision,order", [
-    (HELM, engine.FP64, 17), (LAP, engine.FP64, 18), (HELM, engine.FP32, 19), (HELM, engine.FP32, 20),
-    (HELM, engine.FP32, 24)])
+    (HELM, engine.FP64, 17), (LAP, engine.FP64, 17), (LAP, engine.FP64, 18), (LAP, engine.FP32, 17),
+    (LAP, engine.FP32, 20), (LAP, engine.FP32, 21), (LAP, engine.FP32, 24), (HELM, engine.FP32, 17),
+    (HELM, engine.FP32, 18), (HELM, engine.FP32, 19), (HELM, engine.FP32, 20), (HELM, engine.FP32, 24)])
 def test_high_orders(problem, precision, order):
-    p = _problem(problem, order, 2, 1009, False, 25.0)
+    # (k: the FP32 tables of order 24 within their range at level 3)
+    p = _problem(problem, order, 3, 3001, False, 40.0)
     want, _ = _locals(p, precision, 0)
-    got, _ = _locals(p, precision, 3)
+    got, _ = _locals(p, precision, 5)
     tol = 1e-12 if precision == engine.FP64 else 2e-5
     for a, b in zip(got, want):
         assert np.linalg.norm(a - b) < tol * np.linalg.norm(b)
@@ -67,7 +71,7 @@ def test_target_lists_and_sparse(problem, precision, tol, order):
     p = _problem(problem, order, 4, 5003, True, 30.0)
     _, (pot, grad) = _locals(p, precision, 0)
     for kw in (dict(skip_empty=True), dict(sparse=True)):
-        _, (f, g) = _locals(p, precision, 3, **kw)
+        _, (f, g) = _locals(p, precision, 5, **kw)
         assert np.linalg.norm(f - pot) < tol * np.linalg.norm(pot)
         assert np.linalg.norm(g - grad) < tol * np.linalg.norm(grad)
 

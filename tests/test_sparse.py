@@ -61,7 +61,7 @@ def case_problem(case):
 def solve(p, precision, sparse, keep=False, mode=3):
     cfg = engine.SolverConfig.from_problem(p, precision, skip_empty=True, sparse=sparse)
     s = engine.Solver(cfg)
-    s.set_m2l_kernel(mode)       # 3: the tile kernel; 1: lanes at low orders, tiles above
+    s.set_m2l_kernel(mode)       # 3: the tile kernel; 1: lanes at low orders, columns above
     s.set_sources(p.xs, p.normals).set_strengths(p.q, p.dipoles).set_targets(p.xt).run()
     out = s.field()
     if keep:

@@ -401,6 +401,9 @@ int wbfmm_b200_set_m2l_kernel(wbfmm_b200_solver_t* s, int mode) {
   s->set_m2l_kernel(mode);
   return 0;
 }
+int wbfmm_b200_selftest_m2l_form(wbfmm_b200_solver_t* s, int level) {
+  return s && level >= 0 && level <= kMaxDepth ? s->m2l_form[level] : -1;
+}
 int wbfmm_b200_invalidate_operators(wbfmm_b200_solver_t* s) {
   if (!s) return set_error(WBFMM_B200_E_ARG, "null solver");
   s->invalidate_operators();

@@ -151,6 +151,9 @@ struct wbfmm_b200_solver {
   bool own_stream = false;
   int64_t launches = 0;
   double stage_ms[6] = {0, 0, 0, 0, 0, 0};
+  // kernel of each level's last M2L: 0 warp, 2 lanes, 3 tiles, 4 tensor cores,
+  // 5 columns (wbfmm_b200_set_m2l_kernel), -1 none yet
+  std::vector<int> m2l_form = std::vector<int>(wbfmm::kMaxDepth + 1, -1);
   virtual int set_sources(int, const double*, int, const double*, int, int) = 0;
   virtual int set_strengths(const double*, int, const double*, int, int) = 0;
   virtual int set_targets(int, const double*, int, int) = 0;
@@ -265,7 +268,7 @@ struct Solver : public wbfmm_b200_solver {
   DBuf<T> partial;
   DBuf<unsigned char> lin;         // M2L lane kernel: transposed sources
   DBuf<T> lanes_part;              // and its split partial sums
-  int m2l_mode = 1;                // 0 warp per target, 1 automatic, 2 lanes, 3 tiles
+  int m2l_mode = 1;                // wbfmm_b200_set_m2l_kernel
   int64_t lanes_ctas = 1200;       // lane kernel: split offsets below this many CTAs
   bool tree_only = false;          // structure only: no coefficient arrays
   int eval_field = 3;              // fields evaluate() computes
@@ -876,12 +879,8 @@ struct Solver : public wbfmm_b200_solver {
                                : lanes_supported<T, false>(x.Nin, x.Nout);
     const bool tiles_ok = helm ? tiles_supported<T, true>(x.Nin, x.Nout)
                                : tiles_supported<T, false>(x.Nin, x.Nout);
-    // (level 2 of an FP64 Laplace solve keeps the tiles from order 10 on: 8
-    // targets of a type fill half of its columns' number pairs; 0.121 against
-    // 0.110 ms at p = 14)
     const bool cols_ok = helm ? cols_supported<T, true>(x.Nin, x.Nout)
-                              : cols_supported<T, false>(x.Nin, x.Nout) &&
-                                    !(level == 2 && sizeof(T) == 8 && x.Nin >= 10);
+                              : cols_supported<T, false>(x.Nin, x.Nout);
     // automatic: lanes at the orders where their unrolled code wins, column
     // products above (tiles beyond their orders), the warp-per-target kernel
     // for what none covers.  Lanes / columns, ms on 32768 boxes: Helmholtz
@@ -895,28 +894,38 @@ struct Solver : public wbfmm_b200_solver {
     const int lanes_max = level > 2        ? (helm ? 6 : 8)
                           : sizeof(T) == 8 ? 4
                                            : (helm ? 5 : 8);
-    bool use_tiles = false, use_lanes = false;
+    // (level 2 of a dense FP64 Laplace solve keeps the tiles from order 10 on:
+    // 8 targets of a type fill half of its columns' number pairs; 0.121
+    // against 0.110 ms at p = 14)
+    const bool cols_best = cols_ok && (helm || level > 2 || sizeof(T) == 4 || x.Nin < 10);
+    bool use_cols = false, use_tiles = false, use_lanes = false;
     const int he = helm ? helm_e[level] : 0;
-    if (cfg.sparse) return m2l_sparse(level, x, he, tiles_ok, lanes_ok, lanes_max);
+    if (cfg.sparse) return m2l_sparse(level, x, he, tiles_ok, lanes_ok, cols_ok, lanes_max);
     // tensor cores: Laplace, FP32, equal orders up to (p+1)^2 = 256, mode 4
     if (!helm && sizeof(T) == 4 && m2l_mode == 4 && tc_lap_supported(x.Nin, x.Nout))
       return m2l_tc(level, x);
     if (he) {
-      // the scaled Helmholtz M2L (FP32 tables out of range unscaled) runs
-      // in the tile kernel only
-      if (!tiles_ok)
+      // the scaled Helmholtz M2L (FP32 tables out of range unscaled) runs as
+      // columns or tiles only
+      if (!tiles_ok && !cols_ok)
         return set_error(WBFMM_B200_E_ORDER, "FP32 Helmholtz M2L out of range at this order; use the FP64 form");
-      use_tiles = true;
+      use_cols = cols_ok && !(m2l_mode == 3 && tiles_ok);
+      use_tiles = !use_cols;
     } else if (m2l_mode == 1) {
       use_lanes = lanes_ok && x.Nin <= lanes_max;
-      use_tiles = !use_lanes && tiles_ok;
+      use_cols = !use_lanes && cols_best;
+      use_tiles = !use_lanes && !use_cols && tiles_ok;
     } else if (m2l_mode == 2) {
       use_lanes = lanes_ok;
-      use_tiles = !use_lanes && cols_ok;
+      use_cols = !use_lanes && cols_ok;
     } else if (m2l_mode == 3) {
       use_tiles = tiles_ok;
+    } else if (m2l_mode == 5) {
+      use_cols = cols_ok;
+      use_tiles = !use_cols && tiles_ok;
     }
-    if (use_tiles && cols_ok) return m2l_cols(level, x, he);
+    if (use_cols) return m2l_cols(level, x, he);
+    m2l_form[level] = use_tiles ? 3 : use_lanes ? 2 : 0;
     if (use_tiles) {
       // offset-major target tiles on the transposed singular expansions
       WBFMM_TRY(lin.alloc(lanes_lin_bytes(level, x.Nin, helm, sizeof(T))));
@@ -1031,6 +1040,7 @@ struct Solver : public wbfmm_b200_solver {
   // The M2L of a level as matrix products on columns of target boxes
   // (m2l_cols.cu), dense or on sparse storage
   int m2l_cols(int level, const XlateParams<T>& x, int he) {
+    m2l_form[level] = 5;
     LanesParams<T> lp;
     memset(&lp, 0, sizeof(lp));
     lp.level = level; lp.N = x.Nin;
@@ -1073,24 +1083,24 @@ struct Solver : public wbfmm_b200_solver {
                 : launch_m2l_cols<T, false>(lp, tables, cols_cx.p, cols_tasks.p, stream);
   }
 
-  // The M2L of a level with sparse storage: the lane or tile kernel (the
-  // automatic choice, or the one set with set_m2l_kernel 2 / 3) on compact
-  // transposed sources, one column per stored source group and a zero
+  // The M2L of a level with sparse storage: the lane, column or tile kernel
+  // (the automatic choice, or the one set with set_m2l_kernel 2 / 5 / 3) on
+  // compact transposed sources, one column per stored source group and a zero
   // column, source parents found through the padded-grid slot map, targets
   // from the level's active lists written at their slots
   int m2l_sparse(int level, const XlateParams<T>& x, int he, bool tiles_ok, bool lanes_ok,
-                 int lanes_max) {
+                 bool cols_ok, int lanes_max) {
     bool dense = false;
     const int tc = !tiles_ok ? 0
                    : helm ? tiles_per_cta<T, true>(x.Nin, &dense, true)
                           : tiles_per_cta<T, false>(x.Nin, nullptr, true);
-    bool use_lanes = !he && lanes_ok && (m2l_mode == 2 || (m2l_mode != 3 && x.Nin <= lanes_max));
+    bool use_lanes = !he && lanes_ok &&
+                     (m2l_mode == 2 || (m2l_mode != 3 && m2l_mode != 5 && x.Nin <= lanes_max));
+    if (!use_lanes && cols_ok && !(m2l_mode == 3 && tc > 0)) return m2l_cols(level, x, he);
     if (!use_lanes && tc == 0) use_lanes = !he && lanes_ok;
     if (!use_lanes && tc == 0)
       return set_error(WBFMM_B200_E_ORDER, "sparse level storage: the M2L needs equal orders in [2, 60] at each level");
-    if (!use_lanes && (helm ? cols_supported<T, true>(x.Nin, x.Nout)
-                            : cols_supported<T, false>(x.Nin, x.Nout)))
-      return m2l_cols(level, x, he);
+    m2l_form[level] = use_lanes ? 2 : 3;
     const int64_t G = ngroups[level];
     const int se = helm ? he : x.lap_e;
     WBFMM_TRY(lin.alloc(lanes_lin_groups_bytes(G, x.Nin, helm, sizeof(T))));
@@ -1153,6 +1163,7 @@ struct Solver : public wbfmm_b200_solver {
 
   // The Laplace M2L of a level on the tensor cores (m2l_tc.cu).
   int m2l_tc(int level, const XlateParams<T>& x) {
+    m2l_form[level] = 4;
     LapTcParams lp;
     memset(&lp, 0, sizeof(lp));
     lp.level = level;

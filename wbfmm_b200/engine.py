@@ -115,6 +115,7 @@ def load_library(path: str = LIB_PATH) -> C.CDLL:
         "wbfmm_b200_invalidate_operators": (ip, [vp]),
         "wbfmm_b200_m2l": (ip, [vp, ip]),
         "wbfmm_b200_set_m2l_kernel": (ip, [vp, ip]),
+        "wbfmm_b200_selftest_m2l_form": (ip, [vp, ip]),
         "wbfmm_b200_l2l": (ip, [vp, ip]),
         "wbfmm_b200_direct": (ip, [ip, C.c_double, ip, vp, vp, vp, vp, ip, vp, vp, vp, ip]),
         "wbfmm_b200_fp32_range_ok": (ip, [C.POINTER(Config)]),
@@ -279,9 +280,14 @@ class Solver:
         _check(self.lib.wbfmm_b200_downward_pass(self.h, level))
 
     def set_m2l_kernel(self, mode):
-        """0 warp per target, 1 automatic (default), 2 lane per pair, 3 columns
-        or target tiles; True / False select 1 / 0."""
+        """0 warp per target, 1 automatic (default), 2 lane per pair, 3 target
+        tiles, 4 tensor cores (FP32 Laplace), 5 columns; True / False select
+        1 / 0."""
         _check(self.lib.wbfmm_b200_set_m2l_kernel(self.h, int(mode)))
+
+    def m2l_form(self, level):
+        """Kernel of the level's last M2L, numbered as in set_m2l_kernel."""
+        return int(self.lib.wbfmm_b200_selftest_m2l_form(self.h, int(level)))
 
     def m2l(self, level):
         _check(self.lib.wbfmm_b200_m2l(self.h, level))
