@@ -76,6 +76,17 @@ def test_target_lists_and_sparse(problem, precision, tol, order):
         assert np.linalg.norm(g - grad) < tol * np.linalg.norm(grad)
 
 
+@pytest.mark.parametrize("problem,precision,order,forms", [
+    (LAP, engine.FP32, 12, [4, 4]), (LAP, engine.FP32, 16, [5, 5]), (LAP, engine.FP64, 12, [3, 5]),
+    (HELM, engine.FP32, 4, [2, 2])])
+def test_mode_4_is_automatic_elsewhere(problem, precision, order, forms):
+    p = _problem(problem, order, 3, 1009, False, 25.0)
+    with engine.Solver(engine.SolverConfig.from_problem(p, precision)) as s:
+        s.set_m2l_kernel(4)
+        s.set_sources(p.xs).set_strengths(p.q).set_targets(p.xt).run()
+        assert [s.m2l_form(2), s.m2l_form(3)] == forms
+
+
 FIRST_USE = r"""
 import threading
 import numpy as np

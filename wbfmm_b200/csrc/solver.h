@@ -911,7 +911,7 @@ struct Solver : public wbfmm_b200_solver {
         return set_error(WBFMM_B200_E_ORDER, "FP32 Helmholtz M2L out of range at this order; use the FP64 form");
       use_cols = cols_ok && !(m2l_mode == 3 && tiles_ok);
       use_tiles = !use_cols;
-    } else if (m2l_mode == 1) {
+    } else if (m2l_mode == 1 || m2l_mode == 4) {
       use_lanes = lanes_ok && x.Nin <= lanes_max;
       use_cols = !use_lanes && cols_best;
       use_tiles = !use_lanes && !use_cols && tiles_ok;
