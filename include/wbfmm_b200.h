@@ -205,6 +205,10 @@ int wbfmm_b200_laplace_curl_gradient(wbfmm_b200_solver_t *s, const double *q3,
    (err2[1]) against FP64 sin/cos at the FP32 arguments i * xmax / n,
    i = 0..n. */
 int wbfmm_b200_selftest_sincos(double xmax, int n, double *err2);
+/* Self-test of the FP64 near-field sine and cosine: the largest difference
+   from CUDA's sincos at +-i * xmax / n, i = 0..n, and about every multiple of
+   pi/2 up to xmax (at most 1e6). */
+int wbfmm_b200_selftest_sincos64(double xmax, int n, double *err);
 int wbfmm_b200_synchronize(wbfmm_b200_solver_t *s);
 
 /* Measured FP32 FMA throughput of the current GPU (TFLOP/s, 2 flops per

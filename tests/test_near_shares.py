@@ -99,3 +99,31 @@ def test_infinite_strength(gpu_lib, problem, ns, nt, depth):
                 fields.append(np.concatenate([np.ravel(f) for f in s.field()]))
             assert np.all(np.isinf(fields[1]))
             assert np.array_equal(fields[0], fields[1])
+
+
+# the argument after the reduction is within half a unit of pi/4 (0.9e-16), the
+# series round to about one of 1 (1.5e-16), and CUDA's own values are within 2
+# units (2.2e-16): 5e-16
+@pytest.mark.parametrize("xmax", [3.2, 1e3, 1e5, 1.6e5])     # (the library's above 1e5)
+def test_fp64_sincos(gpu_lib, xmax):
+    assert engine.selftest_sincos64(xmax, 200_000) <= 5e-16
+
+
+# many wavelengths between the points (k r to 2e4 and, where the library's
+# sincos takes over, 2.6e5): r is a few roundings off on either side, k r
+# times 1e-15, and so is the phase
+@pytest.mark.parametrize("k", [3e3, 3e4, 4e5])
+def test_near_high_wavenumber(gpu_lib, k):
+    rng = np.random.default_rng(5)
+    ns, nt = 129, 520
+    xs, xt = rng.uniform(0.01, 0.24, (ns, 3)), rng.uniform(0.01, 0.24, (nt, 3))
+    xs[:, 0] += 0.255 * (np.arange(ns) % 2)
+    q = rng.uniform(0.5, 1.0, (ns, 2))
+    cfg = engine.SolverConfig(engine.HELMHOLTZ, 2, [0, 8, 8], [0, 8, 8], k, (-0.51,) * 3, 1.02,
+                              engine.FP64, engine.POTENTIAL | engine.GRADIENT)
+    with engine.Solver(cfg) as s:
+        pot, grad = s.set_sources(xs).set_strengths(q.ravel()).set_targets(xt).run().field()
+    P, G = _direct(engine.HELMHOLTZ, k, xs, q[:, 0] + 1j * q[:, 1], None, None, xt)
+    tol = 1e-15 * k * np.linalg.norm(xt[:, None] - xs[None], axis=2).max()
+    assert np.linalg.norm(pot[0::2] + 1j * pot[1::2] - P) <= tol * np.linalg.norm(P)
+    assert np.linalg.norm(grad[0::2] + 1j * grad[1::2] - G.ravel()) <= tol * np.linalg.norm(G)

@@ -174,6 +174,7 @@ int launch_narrow(const double* src, float* dst, int64_t n, cudaStream_t s);
 int launch_add_widened(double* dst, const float* src, int64_t n, cudaStream_t s);
 // self-test of the FP32 near-field sine/cosine (kernels.cu)
 int sincos_near_errors(double xmax, int n, double* host_err);
+int sincos_near64_error(double xmax, int n, double* host_err);
 // sparse level storage (sparse.cu): the group map of a level from the n
 // boxes of the level above (stored: box_n != 0 or tmask set; tmask may be
 // null): gmap[g] = slot or kNoGroup, *count = stored groups (device);

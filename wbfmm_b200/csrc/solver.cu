@@ -298,6 +298,12 @@ int wbfmm_b200_selftest_sincos(double xmax, int n, double* err2) {
   if (wbfmm_b200_device_count() < 1) return set_error(WBFMM_B200_E_NOGPU, "no CUDA device is available");
   return sincos_near_errors(xmax, n, err2);
 }
+int wbfmm_b200_selftest_sincos64(double xmax, int n, double* err) {
+  if (!err || n < 1 || !(xmax > 0 && xmax <= 1e6))
+    return set_error(WBFMM_B200_E_ARG, "bad self-test arguments");
+  if (wbfmm_b200_device_count() < 1) return set_error(WBFMM_B200_E_NOGPU, "no CUDA device is available");
+  return sincos_near64_error(xmax, n, err);
+}
 int wbfmm_b200_set_deferred_checks(wbfmm_b200_solver_t* s, int on) {
   SOLVER_CALL(s->set_deferred_checks(on));
 }

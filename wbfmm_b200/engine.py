@@ -94,6 +94,7 @@ def load_library(path: str = LIB_PATH) -> C.CDLL:
         "wbfmm_b200_wait": (ip, [vp]),
         "wbfmm_b200_set_deferred_checks": (ip, [vp, ip]),
         "wbfmm_b200_selftest_sincos": (ip, [C.c_double, ip, dp]),
+        "wbfmm_b200_selftest_sincos64": (ip, [C.c_double, ip, dp]),
         "wbfmm_b200_fp32_fma_peak": (ip, [dp]),
         "wbfmm_b200_error_norms": (ip, [C.c_int64, vp, vp, ip, dp]),
         "wbfmm_b200_laplace_curl": (ip, [vp, vp, ip, vp, ip]),
@@ -463,6 +464,14 @@ def selftest_sincos(xmax: float, n: int):
     err = (C.c_double * 2)()
     _check(load_library().wbfmm_b200_selftest_sincos(float(xmax), int(n), err))
     return float(err[0]), float(err[1])
+
+
+def selftest_sincos64(xmax: float, n: int = 100000) -> float:
+    """Largest difference of the engine's FP64 near-field sin/cos from CUDA's
+    sincos at +-i xmax / n and about the multiples of pi/2 up to xmax."""
+    err = C.c_double()
+    _check(load_library().wbfmm_b200_selftest_sincos64(float(xmax), int(n), C.byref(err)))
+    return float(err.value)
 
 
 def fp32_fma_peak() -> float:
