@@ -254,22 +254,35 @@ __global__ void k_p2m(P2MParams<T> p, int legt, int share) {
   }
 }
 
+constexpr int kP2MWarps = 4;
+
+// lanes per leaf box: 8, 32 or (the warps of a CTA sharing it) 128
 template <typename T, bool HELM>
-int launch_p2m(const P2MParams<T>& p, cudaStream_t s) {
-  if (p.nbox <= 0) return 0;
-  const int nw = 4;
-  const size_t leg = leg_table_bytes<T>(p.N);
-  const size_t rows = p2m_row_bytes<T>(p.N, nw * 32);
-  const size_t one = sizeof(T) * (size_t)nw * ncoef(p.N) * (HELM ? 2 : 1);   // a box per warp
+int p2m_lanes(int N, int64_t nbox, int64_t npts, bool skewed) {
+  const size_t leg = leg_table_bytes<T>(N);
+  const size_t rows = p2m_row_bytes<T>(N, kP2MWarps * 32);
+  const size_t one = sizeof(T) * (size_t)kP2MWarps * ncoef(N) * (HELM ? 2 : 1);   // a box per warp
   // leaves of up to 12 points on average: four boxes per warp (in turn where
   // their counts differ much: clustered points, 2375 in 512 leaves, Laplace
   // order 15 with dipoles, took 3.1 ms against 1.9 without that), while their
-  // accumulators leave room for a second CTA; not where most boxes are empty
+  // accumulators leave room for a second CTA (the rows counted wherever they
+  // are); not where most boxes are empty
   // and the others full (surface points, 33 per occupied leaf: 4.2 ms against
   // 3.1), and not below 24 boxes per SM, which a warp each does not fill: there
   // the longest warp counts (8^3 boxes of clustered points: 2.2 ms against 1.9)
-  const bool few = !p.skewed && p.nbox >= 148 * 24 && p.npts <= 12 * p.nbox && leg + rows + 4 * one <= 100 * 1024;
-  const bool share = !few && p.nbox <= 148 * 8 && p.npts > 48 * p.nbox;
+  if (!skewed && nbox >= 148 * 24 && npts <= 12 * nbox && leg + rows + 4 * one <= 100 * 1024) return 8;
+  return nbox <= 148 * 8 && npts > 48 * nbox ? 128 : 32;
+}
+
+template <typename T, bool HELM>
+int launch_p2m(const P2MParams<T>& p, cudaStream_t s) {
+  if (p.nbox <= 0) return 0;
+  const int nw = kP2MWarps;
+  const size_t leg = leg_table_bytes<T>(p.N);
+  const size_t rows = p2m_row_bytes<T>(p.N, nw * 32);
+  const size_t one = sizeof(T) * (size_t)nw * ncoef(p.N) * (HELM ? 2 : 1);
+  const int lanes = p2m_lanes<T, HELM>(p.N, p.nbox, p.npts, p.skewed != 0);
+  const bool few = lanes == 8, share = lanes == 128;
   auto go = [&](auto srows, auto nc, auto group) -> int {
     constexpr bool SR = decltype(srows)::value;
     constexpr int NC = decltype(nc)::value, G = decltype(group)::value;
@@ -510,6 +523,7 @@ int launch_l2p(const EvalParams<T>& p, cudaStream_t s) {
 
 // ------------------------------------------------------ instantiations
 #define WBFMM_INST(T, H)                                                      \
+  template int p2m_lanes<T, H>(int, int64_t, int64_t, bool);                  \
   template int launch_p2m<T, H>(const P2MParams<T>&, cudaStream_t);          \
   template int launch_l2p<T, H>(const EvalParams<T>&, cudaStream_t);
 WBFMM_INST(double, true)

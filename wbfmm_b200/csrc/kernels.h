@@ -133,6 +133,9 @@ inline int helm_m2l_exp(double k, double w, int P) {
 
 template <typename T, bool HELM>
 int launch_p2m(const P2MParams<T>& p, cudaStream_t s);
+// lanes that it gives a leaf box: 8, 32 or 128
+template <typename T, bool HELM>
+int p2m_lanes(int N, int64_t nbox, int64_t npts, bool skewed);
 template <typename T, bool HELM>
 int launch_m2m(const XlateParams<T>& p, const OpTables<T>& t, cudaStream_t s);
 template <typename T, bool HELM>
