@@ -127,3 +127,32 @@ def test_near_high_wavenumber(gpu_lib, k):
     tol = 1e-15 * k * np.linalg.norm(xt[:, None] - xs[None], axis=2).max()
     assert np.linalg.norm(pot[0::2] + 1j * pot[1::2] - P) <= tol * np.linalg.norm(P)
     assert np.linalg.norm(grad[0::2] + 1j * grad[1::2] - G.ravel()) <= tol * np.linalg.norm(G)
+
+
+# FP64 potentials round the sum once per term: as far from the exact sum as a
+# plain FP64 sum in the same order (over 4000 terms of one sign the sum's
+# roundings are all that counts, and two per term would be sqrt(2) of it; the
+# spread of the mean over 256 values is about 5%)
+def test_fp64_sum(gpu_lib):
+    rng = np.random.default_rng(8)
+    ns, nt, k = 4000, 128, 2.0
+    xs, xt = rng.uniform(0.01, 0.24, (ns, 3)), rng.uniform(0.01, 0.24, (nt, 3))
+    q = rng.uniform(0.5, 1.0, (ns, 2))
+    cfg = engine.SolverConfig(engine.HELMHOLTZ, 2, [0, 8, 8], [0, 8, 8], k, (-0.51,) * 3, 1.02,
+                              engine.FP64, engine.POTENTIAL)
+    with engine.Solver(cfg) as s:
+        pot = s.set_sources(xs).set_strengths(q.ravel()).set_targets(xt).run().field()[0]
+        order = s.tree(2)[0]
+
+    def terms(T):
+        d = xt.astype(T)[:, None] - xs.astype(T)[None, order]
+        kr = T(k) * np.sqrt((d * d).sum(2))
+        a, b = np.sin(kr) / kr, -np.cos(kr) / kr
+        qr, qi = q[order].astype(T).T
+        return np.stack((a * qr - b * qi, b * qr + a * qi), 2)
+
+    exact = terms(np.longdouble).sum(1)
+    plain = np.cumsum(terms(np.float64), axis=1)[:, -1]
+    err = [np.linalg.norm((f - exact).astype(float))
+           for f in (4 * np.pi * pot.reshape(nt, 2).astype(np.longdouble), plain)]
+    assert err[0] <= 1.2 * err[1]

