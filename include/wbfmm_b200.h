@@ -209,11 +209,9 @@ int wbfmm_b200_selftest_sincos(double xmax, int n, double *err2);
    from CUDA's sincos at +-i * xmax / n, i = 0..n, and about every multiple of
    pi/2 up to xmax (at most 1e6). */
 int wbfmm_b200_selftest_sincos64(double xmax, int n, double *err);
-/* Lanes that the leaf expansions of `points` sources in `boxes` leaf boxes
-   give each box: 8, 32, or 128 where a CTA's warps share it (for tests of the
-   forms; skewed: dense storage with skip_empty). */
-int wbfmm_b200_selftest_p2m_lanes(int problem, int precision, int order,
-                                  int64_t boxes, int64_t points, int skewed);
+/* Lanes that the leaf expansions of the sources in place give each leaf box: 8,
+   32, or 128 where a CTA's warps share it (for tests of the forms). */
+int wbfmm_b200_selftest_p2m_form(wbfmm_b200_solver_t *s, int *lanes);
 int wbfmm_b200_synchronize(wbfmm_b200_solver_t *s);
 
 /* Measured FP32 FMA throughput of the current GPU (TFLOP/s, 2 flops per

@@ -59,6 +59,21 @@ def test_flops_per_pair_closed_forms(p):
     assert bench.lap_flops_per_pair(p) == 2 * 2 * R + 2 * X
 
 
+@pytest.mark.parametrize("p", range(0, 21))
+@pytest.mark.parametrize("helm", [False, True])
+def test_flops_per_pair_even_odd(p, helm):
+    """In the even / odd basis: per degree and rotation the blocks over
+    m, nu = 0..n (even) and 1..n (odd), products of a real number with a real
+    (Laplace) or complex one (Helmholtz); the coaxial products as above."""
+    R = sum(1 for n in range(p + 1) for m in range(n + 1) for nu in range(n + 1))
+    R += sum(1 for n in range(p + 1) for m in range(1, n + 1) for nu in range(1, n + 1))
+    X = sum((p + 1 - abs(m)) ** 2 for m in range(-p, p + 1))
+    want = 2 * 4 * R + 8 * X if helm else 2 * 2 * R + 2 * X
+    assert bench.m2l_flops_per_pair(p, helm, 5) == bench.m2l_flops_per_pair(p, helm, 2) == want
+    full = bench.helm_flops_per_pair(p) if helm else bench.lap_flops_per_pair(p)
+    assert bench.m2l_flops_per_pair(p, helm, 3) == full
+
+
 @pytest.mark.parametrize("path, total", [
     (bench.TILE_PROFILE, 71.904256e6 + 5.196288e6),
     (bench.TILE_HELM_PROFILE, 11.853056e6),

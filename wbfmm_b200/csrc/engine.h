@@ -88,11 +88,13 @@ void launch_set_words(uint32_t* a, uint32_t va, uint32_t* b, uint32_t vb,
 // keys[i] = Morton key of point i (src/boxes.c:324-339); vals[i] = i (neither
 // where keys is null); with bad non-null the strict-interior domain check of the sources
 // (src/boxes.c:148-153): *bad = min(*bad, first point outside).
+// stat: leaf counts set to zero for launch_refine_levels.
 // f32: in FP32 arithmetic, as the single-precision build (the *_f API), on
 // coordinates, origin and width that are FP32 values
 void launch_point_keys(const double* pts, int64_t pstr, int n,
                        const double* x0, double D, uint64_t* keys,
-                       uint32_t* vals, int* bad, cudaStream_t s, bool f32 = false);
+                       uint32_t* vals, int* bad, cudaStream_t s, bool f32 = false,
+                       uint32_t* stat = nullptr);
 // target leaf boxes by floor((x-x0)/wb) (src/boxes.c:585-634); vals[i] = i;
 // points outside the closed cube set *bad (host-visible flag) to 1
 void launch_target_keys(const double* pts, int64_t pstr, int n,
@@ -115,13 +117,15 @@ void radix_scratch_free(RadixScratch* scr);
 int launch_curl_combine(const double* g, int nt, double* curl, cudaStream_t s);
 
 // box {i, n} of levels 0..depth from the sorted keys, as `depth` calls of
-// wbfmm_tree_refine leave them (src/boxes.c:208-277)
+// wbfmm_tree_refine leave them (src/boxes.c:208-277); of the leaves also
+// stat[0] = max(stat[0], how many of 16, 32 and 128 the fullest leaf's points
+// exceed), stat[1] += the groups of four consecutive leaves that hold points
 struct LevelBoxes {
   uint32_t* i[kMaxDepth + 1];
   uint32_t* n[kMaxDepth + 1];
 };
 void launch_refine_levels(const uint64_t* sorted_keys, int npts, int depth, const LevelBoxes& b,
-                          cudaStream_t s);
+                          uint32_t* stat, cudaStream_t s);
 // per-box start / count of sorted box ids (plain lower bounds; used for
 // the target bins)
 void launch_box_ranges(const uint64_t* sorted_ids, int n, int level,

@@ -110,6 +110,7 @@ static size_t l2p_row_bytes(int N, bool helm, bool grad, int threads) {
 // orders, FP64) the rows stay in per-thread local arrays, where occupancy
 // is worth more than the shorter latency
 constexpr size_t kRowSmemMax = 48 * 1024;
+constexpr int kP2MWarps = 4;     // per CTA
 constexpr int kL2PBoxes = 4;     // leaf boxes whose expansions an L2P CTA stages
 constexpr int kFixedOrder = 14;   // P2M / L2P order with a compile-time instantiation
 #define WBFMM_TRY_K(call)          \
@@ -123,24 +124,44 @@ constexpr int kFixedOrder = 14;   // P2M / L2P order with a compile-time instant
 // in a per-thread array whose every index the unrolled recursion knows, so
 // that they stay in registers.
 // A warp takes 32 / G boxes, G lanes each: with a few points per leaf a whole
-// warp per box leaves most lanes idle.  The grid is what the SMs hold, each
-// CTA walking over the boxes, so that the recursion constants (square roots
-// and divisions) are formed once per CTA and not once per four boxes (the
-// 262144 leaves of 1e6 points, FP64 Helmholtz p = 6: 2.88 ms with a CTA per
-// four leaves and a warp per leaf, 0.84 so).
+// warp per box leaves most lanes idle (2.5e5 points in 32768 leaves, FP64
+// Helmholtz p = 8: 0.54 ms with a warp per box, 0.28 with 8 lanes).  At G = 32
+// each warp has one box and the SMs take the CTAs as they get free, so that
+// full boxes hold up no others; at G = 8, whose boxes hold 32 points at most,
+// the grid is what the SMs hold, each warp walking over the boxes, and the
+// recursion constants (square roots and divisions) are formed once per CTA.
 // share (G = 32): the warps of a CTA share a box and their sums are added in
 // warp order, for trees of fewer boxes than the SMs have warps.
+// p.stat: of two launches, with G = 8 and with G = 32, one runs (p2m_few).
+// (The block size named to the compiler: without it, it took 64 registers for
+// FP32 Laplace, with it 117: 0.057 -> 0.054 ms on 60000 points in 32768 leaves
+// at order 8, 0.109 -> 0.099 at order 14.)
 template <typename T, bool HELM, bool SROWS, int NC, int G>
-__global__ void k_p2m(P2MParams<T> p, int legt, int share) {
+__global__ void __launch_bounds__(kP2MWarps * 32) k_p2m(P2MParams<T> p, int legt, int share) {
   extern __shared__ __align__(16) unsigned char smraw[];
   constexpr int NG = 32 / G;
+  if (p.stat && p2m_few(p.stat) != (G == 8)) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gl = lane & (G - 1);
   const int nw = blockDim.x >> 5;
-  // Legendre recursion constants of degrees <= N + 2, once per CTA
+  int64_t c0 = share ? (int64_t)blockIdx.x : ((int64_t)blockIdx.x * nw + warp) * NG;
+  // the box's storage index, and (sparse storage) its Morton index
+  int64_t cb, b;
+  uint32_t cnt, start;
+  bool in;
+  auto box = [&]() {
+    cb = c0 + lane / G;
+    in = cb < p.nbox;
+    b = !in ? 0 : p.glist ? (((int64_t)p.glist[cb >> 3] << 3) | (cb & 7)) : cb;
+    cnt = in ? p.box_n[b] : 0;
+    start = in ? p.box_i[b] : 0;
+  };
+  box();
+  // Legendre recursion constants of degrees <= N + 2, once per CTA (not where
+  // its boxes are empty)
   const int LW = (NC > 0 ? NC : p.N) + 3;
   T* lt = (T*)smraw;
   if (legt) {
-    leg_table_fill(lt, LW - 1, threadIdx.x, blockDim.x);
+    if (G == 8 || __syncthreads_or(cnt > 0)) leg_table_fill(lt, LW - 1, threadIdx.x, blockDim.x);
     __syncthreads();
   }
   const int N = NC > 0 ? NC : p.N;
@@ -154,13 +175,7 @@ __global__ void k_p2m(P2MParams<T> p, int legt, int share) {
   T* acc = rows + (SROWS && NC == 0 ? p2m_rows() * RL * blockDim.x : 0) +
            (size_t)(warp * NG + lane / G) * nc * w;
 #pragma unroll 1
-  for (int64_t c0 = share ? (int64_t)blockIdx.x : ((int64_t)blockIdx.x * nw + warp) * NG; c0 < p.nbox;
-       c0 += share ? (int64_t)gridDim.x : (int64_t)gridDim.x * nw * NG) {
-    // the box's storage index, and (sparse storage) its Morton index
-    const int64_t cb = c0 + lane / G;
-    const bool in = cb < p.nbox;
-    const int64_t b = !in ? 0 : p.glist ? (((int64_t)p.glist[cb >> 3] << 3) | (cb & 7)) : cb;
-    const uint32_t cnt = in ? p.box_n[b] : 0, start = in ? p.box_i[b] : 0;
+  while (c0 < p.nbox) {
     const uint32_t most = NG == 1 ? cnt : __reduce_max_sync(0xffffffffu, cnt);
     if (most > 0) {
       for (int c = gl; c < nc * w; c += G) acc[c] = T(0);
@@ -227,18 +242,13 @@ __global__ void k_p2m(P2MParams<T> p, int legt, int share) {
       }
       __syncwarp();
     }
-    if (share) {
-      if (most > 0) {
-        __syncthreads();     // (the box is the CTA's)
-        if (warp == 0)
-          for (int c = lane; c < nc * w; c += 32)
-            for (int u = 1; u < nw; u++) acc[c] += acc[c + u * nc * w];
-        __syncwarp();
-      }
-      if (warp) {
-        if (most > 0) __syncthreads();
-        continue;
-      }
+    if (share) {             // (the CTA's only box)
+      if (most > 0) __syncthreads();
+      if (warp) return;
+      if (most > 0)
+        for (int c = lane; c < nc * w; c += 32)
+          for (int u = 1; u < nw; u++) acc[c] += acc[c + u * nc * w];
+      __syncwarp();
     }
     // (a box without points beside one with points holds zeros)
     for (int c = gl; in && c < nc; c += G) {
@@ -249,28 +259,30 @@ __global__ void k_p2m(P2MParams<T> p, int legt, int share) {
         else p.mps[w * o + u] = v;
       }
     }
-    if (share && most > 0) __syncthreads();
-    else __syncwarp();
+    if (G == 32) break;
+    __syncwarp();
+    c0 += (int64_t)gridDim.x * nw * NG;
+    box();
   }
 }
 
-constexpr int kP2MWarps = 4;
-
 // lanes per leaf box: 8, 32 or (the warps of a CTA sharing it) 128
 template <typename T, bool HELM>
-int p2m_lanes(int N, int64_t nbox, int64_t npts, bool skewed) {
+int p2m_lanes(int N, int64_t nbox, int64_t npts) {
   const size_t leg = leg_table_bytes<T>(N);
   const size_t rows = p2m_row_bytes<T>(N, kP2MWarps * 32);
   const size_t one = sizeof(T) * (size_t)kP2MWarps * ncoef(N) * (HELM ? 2 : 1);   // a box per warp
-  // leaves of up to 12 points on average: four boxes per warp (in turn where
-  // their counts differ much: clustered points, 2375 in 512 leaves, Laplace
-  // order 15 with dipoles, took 3.1 ms against 1.9 without that), while their
-  // accumulators leave room for a second CTA (the rows counted wherever they
-  // are); not where most boxes are empty
-  // and the others full (surface points, 33 per occupied leaf: 4.2 ms against
-  // 3.1), and not below 24 boxes per SM, which a warp each does not fill: there
-  // the longest warp counts (8^3 boxes of clustered points: 2.2 ms against 1.9)
-  if (!skewed && nbox >= 148 * 24 && npts <= 12 * nbox && leg + rows + 4 * one <= 100 * 1024) return 8;
+  // leaves of up to 12 points on average, 96 per SM, or of up to 6, 24 per SM
+  // (not at order 14, whose form with a warp per box is unrolled): four boxes
+  // per warp, while their accumulators leave room for a second CTA (the rows
+  // counted wherever they are) and the leaves' counts allow (p2m_few).  FP64
+  // Laplace p = 8, ms with a warp per box / 8 lanes: 32768 uniform leaves of 7.6
+  // points 0.23 / 0.15, 4096 of 2 0.043 / 0.036, 4096 of 11 0.045 / 0.047; of
+  // clustered points, 8 lanes throughout: 4096 leaves of 11 0.28 / 0.82
+  const bool many = nbox >= 4 * 148 * 24, fixed = N == kFixedOrder && !(HELM && sizeof(T) == 8);
+  if (nbox >= 148 * 24 && (many || !fixed) && npts <= (many ? 12 : 6) * nbox &&
+      leg + rows + 4 * one <= 100 * 1024)
+    return 8;
   return nbox <= 148 * 8 && npts > 48 * nbox ? 128 : 32;
 }
 
@@ -281,18 +293,19 @@ int launch_p2m(const P2MParams<T>& p, cudaStream_t s) {
   const size_t leg = leg_table_bytes<T>(p.N);
   const size_t rows = p2m_row_bytes<T>(p.N, nw * 32);
   const size_t one = sizeof(T) * (size_t)nw * ncoef(p.N) * (HELM ? 2 : 1);
-  const int lanes = p2m_lanes<T, HELM>(p.N, p.nbox, p.npts, p.skewed != 0);
+  const int lanes = p2m_lanes<T, HELM>(p.N, p.nbox, p.npts);
   const bool few = lanes == 8, share = lanes == 128;
   auto go = [&](auto srows, auto nc, auto group) -> int {
     constexpr bool SR = decltype(srows)::value;
     constexpr int NC = decltype(nc)::value, G = decltype(group)::value;
     const size_t smem = leg + (SR ? rows : 0) + one * (32 / G);
     if (smem > 48 * 1024) WBFMM_SMEM(smem, k_p2m<T, HELM, SR, NC, G>);
-    // at most 8 CTAs per SM: about what registers and shared memory hold
-    const int64_t need = (p.nbox + nw * (32 / G) - 1) / (nw * (32 / G));
-    const unsigned grid = (unsigned)(need < 148 * 8 ? need : 148 * 8);
-    k_p2m<T, HELM, SR, NC, G><<<share ? (unsigned)p.nbox : grid, nw * 32, smem, s>>>(
-        p, leg ? 1 : 0, share ? 1 : 0);
+    P2MParams<T> a = p;
+    if (!few) a.stat = nullptr;
+    // G = 8: at most 8 CTAs per SM, about what registers and shared memory hold
+    const int64_t need = share ? p.nbox : (p.nbox + nw * (32 / G) - 1) / (nw * (32 / G));
+    const unsigned grid = (unsigned)(G == 32 || need < 148 * 8 ? need : 148 * 8);
+    k_p2m<T, HELM, SR, NC, G><<<grid, nw * 32, smem, s>>>(a, leg ? 1 : 0, share ? 1 : 0);
     return 0;
   };
   const std::integral_constant<int, 0> any;
@@ -303,9 +316,8 @@ int launch_p2m(const P2MParams<T>& p, cudaStream_t s) {
   // the serving orders' leaf expansions: rows in registers (not for FP64
   // Helmholtz, whose unrolled recursion exceeds the register file)
   constexpr bool kFixedOk = !(HELM && sizeof(T) == 8);
-  if (few) {
-    WBFMM_TRY_K(rows <= kRowSmemMax ? go(yes, any, eighth) : go(no, any, eighth));
-  } else if (kFixedOk && p.N == kFixedOrder) {
+  if (few) WBFMM_TRY_K(rows <= kRowSmemMax ? go(yes, any, eighth) : go(no, any, eighth));
+  if (kFixedOk && p.N == kFixedOrder) {
     if constexpr (kFixedOk) WBFMM_TRY_K(go(no, std::integral_constant<int, kFixedOrder>(), whole));
   } else {
     WBFMM_TRY_K(rows <= kRowSmemMax ? go(yes, any, whole) : go(no, any, whole));
@@ -523,7 +535,7 @@ int launch_l2p(const EvalParams<T>& p, cudaStream_t s) {
 
 // ------------------------------------------------------ instantiations
 #define WBFMM_INST(T, H)                                                      \
-  template int p2m_lanes<T, H>(int, int64_t, int64_t, bool);                  \
+  template int p2m_lanes<T, H>(int, int64_t, int64_t);                       \
   template int launch_p2m<T, H>(const P2MParams<T>&, cudaStream_t);          \
   template int launch_l2p<T, H>(const EvalParams<T>&, cudaStream_t);
 WBFMM_INST(double, true)

@@ -40,7 +40,7 @@ template <typename T>
 struct P2MParams {
   int64_t nbox;       // boxes at the leaf level
   int64_t npts;       // sources in them
-  int skewed;         // most boxes may be empty (dense storage with skip_empty)
+  const uint32_t* stat;   // what launch_refine_levels counted of the leaves
   int level, N;
   double x0, y0, z0, wb;
   T k;
@@ -133,9 +133,20 @@ inline int helm_m2l_exp(double k, double w, int P) {
 
 template <typename T, bool HELM>
 int launch_p2m(const P2MParams<T>& p, cudaStream_t s);
-// lanes that it gives a leaf box: 8, 32 or 128
+// lanes that it gives a leaf box: 8 (if the leaves' counts allow, p2m_few),
+// 32 or 128
 template <typename T, bool HELM>
-int p2m_lanes(int N, int64_t nbox, int64_t npts, bool skewed);
+int p2m_lanes(int N, int64_t nbox, int64_t npts);
+// launch_refine_levels' words -> whether 8 lanes per leaf box do: no leaf of
+// more than 16 points, or of more than 32 where the occupied groups of four
+// give each SM 24 warps, or of more than 128 where they give it eight times
+// that, so that no warp's boxes take longer than the rest of the tree
+HD bool p2m_few(const uint32_t* stat) {
+  const uint32_t least = 148 * 24;
+  return stat[0] == 0 || (stat[0] == 1 && stat[1] >= least) ||
+         (stat[0] == 2 && stat[1] >= 8 * least);
+}
+
 template <typename T, bool HELM>
 int launch_m2m(const XlateParams<T>& p, const OpTables<T>& t, cudaStream_t s);
 template <typename T, bool HELM>

@@ -215,8 +215,13 @@ ColsPlan cols_plan(int P, int ncol) {
 
 constexpr size_t kColsSmemCap = 227 * 1024;
 
-// columns per lane: the most whose rows fit (fewer table reads per product);
-// level 2 has 8 targets of a type, which 8 columns hold (Laplace FP32 order 14:
+// columns per lane: the most whose rows fit (fewer table reads per product).
+// ms on 4096 boxes with them and with half of them, which two CTAs per SM may
+// then hold: FP32 Helmholtz p = 8 0.63 / 0.81, p = 14 1.60 / 2.17, Laplace
+// p = 10 0.44 / 0.54, p = 14 0.85 / 0.91; FP64 Helmholtz p = 8 1.25 / 1.30,
+// p = 10 1.77 / 1.94, Laplace p = 10 0.90 / 0.94; half are faster at FP64 p = 7
+// (1.04 / 0.93), p = 12 (2.71 / 2.40) and Laplace p = 9 (0.75 / 0.69) only.
+// Level 2 has 8 targets of a type, which 8 columns hold (Laplace FP32 order 14:
 // 0.155 ms with 32 columns, 28 of them idle)
 template <typename T, bool HELM>
 int cols_cpl(int P, int level) {

@@ -257,10 +257,10 @@ struct LaneReg {
 
 // CTAs per SM that the register-resident variant is compiled for (it caps
 // the registers per thread at 65536 / (128 * this)).  Measured on B200, FP32,
-// level-5/6 M2L (ms for caps 3 / 4 / none): Helmholtz p = 6 11.96 / 13.85 /
-// 10.51 (no cap: ILP of the unrolled body beats occupancy), p = 5 0.914 /
-// 0.986 / 0.943; Laplace p = 6 0.863 / 0.756 / 1.048, p = 8 1.694 / 1.837 /
-// 1.781.  WBFMM_LANES_REG_CTAS overrides the table.
+// M2L of 32768 boxes (ms for caps 3 / 4 / none): Helmholtz p = 6 0.968 / 1.160 /
+// 0.963 (262144 boxes: 6.99 / 9.44 / 7.26), p = 5 0.604 / 0.574 / 0.669; Laplace
+// p = 6 0.542 / 0.506 / 0.589, p = 8 0.932 / 0.939 / 1.011.
+// WBFMM_LANES_REG_CTAS overrides the table.
 template <typename T, bool HELM, int P>
 struct LaneRegCtas {
 #ifdef WBFMM_LANES_REG_CTAS

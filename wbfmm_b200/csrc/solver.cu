@@ -304,14 +304,9 @@ int wbfmm_b200_selftest_sincos64(double xmax, int n, double* err) {
   if (wbfmm_b200_device_count() < 1) return set_error(WBFMM_B200_E_NOGPU, "no CUDA device is available");
   return sincos_near64_error(xmax, n, err);
 }
-int wbfmm_b200_selftest_p2m_lanes(int problem, int precision, int order, int64_t boxes,
-                                  int64_t points, int skewed) {
-  const bool helm = problem == WBFMM_B200_HELMHOLTZ, sk = skewed != 0;
-  if (precision == WBFMM_B200_FP32)
-    return helm ? p2m_lanes<float, true>(order, boxes, points, sk)
-                : p2m_lanes<float, false>(order, boxes, points, sk);
-  return helm ? p2m_lanes<double, true>(order, boxes, points, sk)
-              : p2m_lanes<double, false>(order, boxes, points, sk);
+int wbfmm_b200_selftest_p2m_form(wbfmm_b200_solver_t* s, int* lanes) {
+  if (!lanes) return set_error(WBFMM_B200_E_ARG, "null argument");
+  SOLVER_CALL(s->p2m_form(lanes));
 }
 int wbfmm_b200_set_deferred_checks(wbfmm_b200_solver_t* s, int on) {
   SOLVER_CALL(s->set_deferred_checks(on));

@@ -159,6 +159,7 @@ struct wbfmm_b200_solver {
   virtual int set_targets(int, const double*, int, int) = 0;
   virtual int build_operators() = 0;
   virtual int leaf_expansions() = 0;
+  virtual int p2m_form(int* lanes) = 0;
   virtual int upward(int level) = 0;
   virtual int downward(int level) = 0;
   virtual int evaluate() = 0;
@@ -207,6 +208,7 @@ struct Solver : public wbfmm_b200_solver {
   bool have_q = false, have_dip = false, have_normals = false;
   RadixScratch rs;
   DBuf<uint32_t> box_i[kMaxDepth + 1], box_n[kMaxDepth + 1];
+  DBuf<uint32_t> leaf_stat; // launch_refine_levels' counts of the leaves (P2M)
   // coefficients (Layout L; with sparse storage, per stored group)
   DBuf<T> mps[kMaxDepth + 1], mpr[kMaxDepth + 1];
   // sparse level storage (sparse.cu): per level the group -> slot map, the
@@ -297,7 +299,7 @@ struct Solver : public wbfmm_b200_solver {
 
   template <class F>
   void each_buf(F&& f) {
-    f(pts_in); f(nrm_in); f(keys); f(ip); f(sx); f(sy); f(sz);
+    f(pts_in); f(nrm_in); f(keys); f(ip); f(leaf_stat); f(sx); f(sy); f(sz);
     f(snx); f(sny); f(snz); f(sq); f(sdip); f(stage); f(nstage);
     for (int l = 0; l <= kMaxDepth; l++) {
       f(box_i[l]); f(box_n[l]); f(mps[l]); f(mpr[l]); f(tmask[l]);
@@ -455,8 +457,9 @@ struct Solver : public wbfmm_b200_solver {
     xstr = xs_str;
     WBFMM_TRY(keys.alloc(n));
     WBFMM_TRY(ip.alloc(n));
+    WBFMM_TRY(leaf_stat.alloc(2));
     launch_point_keys(dpts, xs_str, n, cfg.x0, cfg.D, keys.p, ip.p,
-                      async_checks ? flag.p : nullptr, stream, cfg.keys_fp32 != 0);
+                      async_checks ? flag.p : nullptr, stream, cfg.keys_fp32 != 0, leaf_stat.p);
     // full 60-bit keys (the reference's point order), or with leaf_order
     // only the bits that select the leaf box
     const int sort_lo = cfg.leaf_order ? 60 - 3 * depth : 0;
@@ -492,7 +495,7 @@ struct Solver : public wbfmm_b200_solver {
       lb.i[l] = box_i[l].p;
       lb.n[l] = box_n[l].p;
     }
-    launch_refine_levels(keys.p, n, depth, lb, stream);
+    launch_refine_levels(keys.p, n, depth, lb, leaf_stat.p, stream);
     launches++;
     WBFMM_CUDA(cudaGetLastError());
     // coefficient arrays (arrays adopted from the caller are kept; sparse
@@ -798,7 +801,7 @@ struct Solver : public wbfmm_b200_solver {
     P2MParams<T> p;
     p.nbox = (int64_t)1 << (3 * depth);
     p.npts = nsrc;
-    p.skewed = cfg.skip_empty && !cfg.sparse;
+    p.stat = leaf_stat.p;
     p.level = depth; p.N = cfg.order_s[depth];
     p.x0 = cfg.x0[0]; p.y0 = cfg.x0[1]; p.z0 = cfg.x0[2]; p.wb = width(depth);
     p.k = (T)cfg.k;
@@ -815,6 +818,19 @@ struct Solver : public wbfmm_b200_solver {
     }
     launches++;
     return helm ? launch_p2m<T, true>(p, stream) : launch_p2m<T, false>(p, stream);
+  }
+
+  int p2m_form(int* lanes) override {
+    if (nsrc <= 0) return set_error(WBFMM_B200_E_STATE, "set_sources first");
+    WBFMM_TRY(prepare_sparse());
+    const int64_t nb = cfg.sparse ? 8 * ngroups[depth] : (int64_t)1 << (3 * depth);
+    *lanes = helm ? p2m_lanes<T, true>(cfg.order_s[depth], nb, nsrc)
+                  : p2m_lanes<T, false>(cfg.order_s[depth], nb, nsrc);
+    uint32_t st[2];
+    WBFMM_CUDA(cudaMemcpyAsync(st, leaf_stat.p, sizeof(st), cudaMemcpyDeviceToHost, stream));
+    WBFMM_CUDA(cudaStreamSynchronize(stream));
+    if (*lanes == 8 && !p2m_few(st)) *lanes = 32;
+    return 0;
   }
 
   XlateParams<T> xparams() const {

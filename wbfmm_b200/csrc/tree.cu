@@ -116,9 +116,10 @@ __device__ __forceinline__ bool outside_open(double x, double x0, double D, bool
 __global__ void k_point_keys(const double* __restrict__ pts, int64_t pstr,
                              int n, double x0, double y0, double z0, double D,
                              uint64_t* __restrict__ keys,
-                             uint32_t* __restrict__ vals, int* bad, bool f32) {
+                             uint32_t* __restrict__ vals, int* bad, bool f32, uint32_t* stat) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
+  if (stat && i == 0) stat[0] = stat[1] = 0;
   const double* p = pts + (int64_t)i * pstr;
   const double x = p[0], y = p[1], z = p[2];
   if (bad && (outside_open(x, x0, D, f32) || outside_open(y, y0, D, f32) ||
@@ -140,10 +141,10 @@ __global__ void k_point_keys(const double* __restrict__ pts, int64_t pstr,
 
 void launch_point_keys(const double* pts, int64_t pstr, int n,
                        const double* x0, double D, uint64_t* keys,
-                       uint32_t* vals, int* bad, cudaStream_t s, bool f32) {
+                       uint32_t* vals, int* bad, cudaStream_t s, bool f32, uint32_t* stat) {
   if (n <= 0) return;
   k_point_keys<<<(n + 255) / 256, 256, 0, s>>>(pts, pstr, n, x0[0], x0[1],
-                                               x0[2], D, keys, vals, bad, f32);
+                                               x0[2], D, keys, vals, bad, f32, stat);
 }
 
 // ------------------------------------------------------------ radix sort
@@ -408,12 +409,8 @@ __device__ __forceinline__ uint32_t lower_bound_box(const uint64_t* keys,
 // and then advances P.i by P.n.  A box that is a first child over several
 // levels takes the i of the highest of those boxes, whose first position is
 // its own: `a`, the ancestor by the trailing zero digits (i = 0 from the root).
-__global__ void k_refine_levels(const uint64_t* __restrict__ keys, int npts, int depth,
-                                LevelBoxes b) {
-  int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int l = 0;
-  while (l <= depth && e >= ((int64_t)1 << (3 * l))) { e -= (int64_t)1 << (3 * l); l++; }
-  if (l > depth) return;
+__device__ __forceinline__ uint32_t refine_box(const uint64_t* __restrict__ keys, int npts,
+                                               int depth, int l, int64_t e, const LevelBoxes& b) {
   const int shift = 3 * (20 - l);
   const uint64_t c = (uint64_t)e;
   const uint32_t lb = lower_bound_box(keys, npts, shift, c);
@@ -428,13 +425,35 @@ __global__ void k_refine_levels(const uint64_t* __restrict__ keys, int npts, int
   }
   b.n[l][e] = ub - lb;
   b.i[l][e] = l < depth ? i + (ub - lb) : i;
+  return ub - lb;
+}
+
+__global__ void k_refine_levels(const uint64_t* __restrict__ keys, int npts, int depth,
+                                LevelBoxes b, uint32_t* stat) {
+  // the leaves first (consecutive ones in a warp), then levels 0, 1, ...
+  int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool leaf = e < ((int64_t)1 << (3 * depth));
+  int l = depth;
+  if (!leaf) {
+    e -= (int64_t)1 << (3 * depth);
+    l = 0;
+    while (l < depth && e >= ((int64_t)1 << (3 * l))) { e -= (int64_t)1 << (3 * l); l++; }
+  }
+  const uint32_t cnt = leaf || l < depth ? refine_box(keys, npts, depth, l, e, b) : 0;
+  uint32_t step = leaf ? (cnt > 16) + (cnt > 32) + (cnt > 128) : 0;
+  step = __reduce_max_sync(0xffffffffu, step);
+  const unsigned held = __ballot_sync(0xffffffffu, leaf && cnt > 0);
+  const int lane = threadIdx.x & 31;
+  const int groups = __syncthreads_count((lane & 3) == 0 && ((held >> lane) & 15));
+  if (lane == 0 && step > *(volatile uint32_t*)stat) atomicMax(stat, step);
+  if (threadIdx.x == 0 && groups) atomicAdd(stat + 1, (uint32_t)groups);
 }
 
 void launch_refine_levels(const uint64_t* sorted_keys, int npts, int depth, const LevelBoxes& b,
-                          cudaStream_t s) {
+                          uint32_t* stat, cudaStream_t s) {
   int64_t tot = 0;
   for (int l = 0; l <= depth; l++) tot += (int64_t)1 << (3 * l);
-  k_refine_levels<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(sorted_keys, npts, depth, b);
+  k_refine_levels<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(sorted_keys, npts, depth, b, stat);
 }
 
 __global__ void k_box_ranges(const uint64_t* __restrict__ ids, int n,

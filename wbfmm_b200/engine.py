@@ -95,7 +95,7 @@ def load_library(path: str = LIB_PATH) -> C.CDLL:
         "wbfmm_b200_set_deferred_checks": (ip, [vp, ip]),
         "wbfmm_b200_selftest_sincos": (ip, [C.c_double, ip, dp]),
         "wbfmm_b200_selftest_sincos64": (ip, [C.c_double, ip, dp]),
-        "wbfmm_b200_selftest_p2m_lanes": (ip, [ip, ip, ip, C.c_int64, C.c_int64, ip]),
+        "wbfmm_b200_selftest_p2m_form": (ip, [vp, C.POINTER(C.c_int)]),
         "wbfmm_b200_fp32_fma_peak": (ip, [dp]),
         "wbfmm_b200_error_norms": (ip, [C.c_int64, vp, vp, ip, dp]),
         "wbfmm_b200_laplace_curl": (ip, [vp, vp, ip, vp, ip]),
@@ -274,6 +274,12 @@ class Solver:
 
     def leaf_expansions(self):
         _check(self.lib.wbfmm_b200_leaf_expansions(self.h))
+
+    def p2m_form(self):
+        """Lanes that leaf_expansions gives each leaf box: 8, 32, or 128 (a CTA)."""
+        lanes = C.c_int()
+        _check(self.lib.wbfmm_b200_selftest_p2m_form(self.h, C.byref(lanes)))
+        return lanes.value
 
     def upward_pass(self, level):
         _check(self.lib.wbfmm_b200_upward_pass(self.h, level))
@@ -473,13 +479,6 @@ def selftest_sincos64(xmax: float, n: int = 100000) -> float:
     err = C.c_double()
     _check(load_library().wbfmm_b200_selftest_sincos64(float(xmax), int(n), C.byref(err)))
     return float(err.value)
-
-
-def selftest_p2m_lanes(problem: int, precision: int, order: int, boxes: int, points: int,
-                       skewed: bool = False) -> int:
-    """Lanes that the leaf expansions give each box: 8, 32, or 128 (a CTA)."""
-    return int(load_library().wbfmm_b200_selftest_p2m_lanes(problem, precision, order, boxes,
-                                                            points, int(skewed)))
 
 
 def fp32_fma_peak() -> float:
