@@ -32,15 +32,14 @@ dataset).  One step = one batch of SERVE_BATCH requests.
   `served_p50_s` / `served_p99_s` / `plain_p50_s` / `plain_p99_s` are at 70%.
 * accuracy: the served fields of sampled requests against the FP64 GPU
   direct sum (itself pinned to the reference's direct sums).
-* `roofline`: the stream's dominant kernel, the FP32 Helmholtz tile M2L
-  (23% of the stream's device time in profiles/launches_serving_stream_48.md)
-  on an order-14 level (1e5 points, k = 10, level 4): algorithmic FLOPs of
-  the dense level's list-4 pairs / event time, against the FP32 FMA peak
-  measured live on the GPU (`wbfmm_b200_fp32_fma_peak`), `traffic` from the
-  committed ncu capture of the same launch.  `roofline_p2p`: the FP32 near
-  field (k_p2p, the next kernel, 18%) on a 2e5-point Helmholtz cube, exact
-  pair count; `roofline_m2l_laplace`: the Laplace tile M2L on an order-14
-  level (3e5 points, level 5).
+* `roofline`: the stream's FP32 Helmholtz M2L (shares of the stream's device
+  time: profiles/launches_serving_stream_48.md) on an order-14 level (1e5
+  points, k = 10, level 4): the FLOPs that its kernel does for the dense
+  level's list-4 pairs / event time, against the FP32 FMA peak measured live
+  on the GPU (`wbfmm_b200_fp32_fma_peak`), `traffic` from the committed ncu
+  capture of the same launch.  `roofline_p2p`: the FP32 near field (k_p2p) on
+  a 2e5-point Helmholtz cube, exact pair count; `roofline_m2l_laplace`: the
+  Laplace M2L on an order-14 level (3e5 points, level 5).
 * `cpu_baseline` and `--impl reference`: the reference's own CPU FMM
   (oracle/_ref, the unmodified reference sources, M2L on up to 16 threads)
   run request by request on a bounded sample of the stream.
@@ -82,6 +81,8 @@ SERVE_LOADS = (0.3, 0.5, 0.7, 0.9)
 CPU_SAMPLE_MAX_N = 20_000
 CPU_SAMPLE_REQUESTS = 12
 TILE_PROFILE = os.path.join(ROOT, "profiles", "k_m2l_tiles_laplace_3e5_p14_level5.md")
+COLS_PROFILE = os.path.join(ROOT, "profiles", "k_m2l_cols_laplace_3e5_p14_level5.md")
+COLS_HELM_PROFILE = os.path.join(ROOT, "profiles", "k_m2l_cols_helmholtz_1e5_p14_level4.md")
 
 
 # ---------------------------------------------------------------- helpers
@@ -153,6 +154,26 @@ def helm_flops_per_pair(p: int) -> int:
     R = (p + 1) * (2 * p + 1) * (2 * p + 3) // 3
     X = (p + 1) ** 2 + p * (p + 1) ** 2 - p * (p + 1) * (p + 2) // 3
     return 2 * 4 * R + 8 * X
+
+
+def even_odd_flops_per_pair(p: int, helm: bool) -> int:
+    """The same shift in the even / odd basis of the lane and column kernels: a
+    rotation is the products of two real blocks, (n+1)^2 and n^2 per degree,
+    the coaxial translation as above (the phases, some 2%, left out)."""
+    R = sum((n + 1) ** 2 + n * n for n in range(p + 1))
+    X = sum((p + 1 - abs(m)) ** 2 for m in range(-p, p + 1))
+    return 2 * 4 * R + 8 * X if helm else 2 * 2 * R + 2 * X
+
+
+# wbfmm_b200_set_m2l_kernel's numbers
+M2L_KERNELS = {0: "k_m2l", 2: "k_m2l_lanes", 3: "k_m2l_tiles", 4: "k_m2l_tc", 5: "k_m2l_cols"}
+
+
+def m2l_flops_per_pair(p: int, helm: bool, form: int) -> int:
+    """FLOPs per pair of the M2L kernel `form`."""
+    if form in (2, 5):
+        return even_odd_flops_per_pair(p, helm)
+    return helm_flops_per_pair(p) if helm else lap_flops_per_pair(p)
 
 
 class ClockSampler:
@@ -300,18 +321,20 @@ def workload(args, rank):
 # with one or two captured launches sees the steady-state launch.
 PROFILE_CASES = """
 
-  m2l_tiles_laplace_p14     Laplace, 3e5 uniform points, depth 5, order 14,
-                            FP32: M2L of level 5 (offset-major tile kernel)
-  m2l_tiles_helmholtz_p14   Helmholtz k = 10, 1e5 points, depth 4, orders
+  m2l_cols_laplace_p14      Laplace, 3e5 uniform points, depth 5, order 14,
+                            FP32: M2L of level 5 (column kernel)
+  m2l_cols_helmholtz_p14    Helmholtz k = 10, 1e5 points, depth 4, orders
                             max(14, kw rule), FP32: M2L of level 4
+  m2l_tiles_laplace_p14, m2l_tiles_helmholtz_p14
+                            the same in the offset-major tile kernel (mode 3)
   m2l_lanes_helmholtz_p6    Helmholtz k = 8, 1e6 points, depth 6, the
                             benchmark's orders, FP32: M2L of level 6
                             (lane-per-pair kernel)
   m2l_lanes_laplace_clusters_p10
                             Laplace, 2e6 points in 8 Gaussian clusters,
                             depth 7, order 10, skip_empty, FP32: M2L of
-                            level 7 (lane kernel on target lists)
-  m2l_tc_laplace_p14        as m2l_tiles_laplace_p14 on the tensor cores
+                            level 7 (lane kernel, mode 2, on target lists)
+  m2l_tc_laplace_p14        as m2l_cols_laplace_p14 on the tensor cores
                             (M2L mode 4: tcgen05 3xTF32)
   p2p_helmholtz             Helmholtz k = 10, 2e5 points, depth 4, FP32:
                             evaluation (L2P + P2P)
@@ -348,28 +371,27 @@ def _cube(problem, n, depth, order, k=0.0, seed=1):
 
 def profile_case(case: str) -> None:
     from wbfmm_b200 import engine, workloads as W
-    if case == "m2l_tiles_laplace_p14":
-        p = _cube(engine.LAPLACE, 300_000, 5, 14)
-        _solve_then(p, engine.FP32, lambda s: s.m2l(5))
-    elif case == "m2l_tc_laplace_p14":
-        p = _cube(engine.LAPLACE, 300_000, 5, 14)
+    def m2l(level):
+        def stage(s):
+            s.set_m2l_kernel({"cols": 5, "tiles": 3, "tc": 4, "lanes": 2}[case.split("_")[1]])
+            s.m2l(level)
+        return stage
 
-        def tc(s):
-            s.set_m2l_kernel(4)
-            s.m2l(5)
-        _solve_then(p, engine.FP32, tc)
+    if case in ("m2l_cols_laplace_p14", "m2l_tiles_laplace_p14", "m2l_tc_laplace_p14"):
+        p = _cube(engine.LAPLACE, 300_000, 5, 14)
+        _solve_then(p, engine.FP32, m2l(5))
     elif case == "target_bases_helmholtz":
         p = _cube(engine.HELMHOLTZ, 200_000, 4, 8, k=10.0)
         _solve_then(p, engine.FP64, lambda s: s.target_bases().evaluate_bases())
-    elif case == "m2l_tiles_helmholtz_p14":
+    elif case in ("m2l_cols_helmholtz_p14", "m2l_tiles_helmholtz_p14"):
         p = _cube(engine.HELMHOLTZ, 100_000, 4, 14, k=10.0)
-        _solve_then(p, engine.FP32, lambda s: s.m2l(4))
+        _solve_then(p, engine.FP32, m2l(4))
     elif case == "m2l_lanes_helmholtz_p6":
         p = W.helmholtz_cube(1_000_000, k=8.0, depth=6, seed=2)
-        _solve_then(p, engine.FP32, lambda s: s.m2l(6))
+        _solve_then(p, engine.FP32, m2l(6))
     elif case == "m2l_lanes_laplace_clusters_p10":
         p = W.laplace_clusters(2_000_000, depth=7, order=10, seed=5)
-        _solve_then(p, engine.FP32, lambda s: s.m2l(7), skip_empty=True)
+        _solve_then(p, engine.FP32, m2l(7), skip_empty=True)
     elif case == "p2p_helmholtz":
         p = _cube(engine.HELMHOLTZ, 200_000, 4, 8, k=10.0)
         _solve_then(p, engine.FP32, lambda s: s.evaluate())
@@ -746,7 +768,7 @@ def single_solve_section(args, ws, rank, local, p, n_acc, acc_seed, skip_empty, 
         ms = dist_max(float(np.mean(step_ms)), ws)
         launches = (s.kernel_launches() - l0) // steps
         stages = s.stage_times()
-        m2l_ms = {}
+        m2l_ms, m2l_form = {}, {}
         for lv in range(2, p.depth + 1):
             a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             with torch.cuda.stream(stream):
@@ -756,9 +778,10 @@ def single_solve_section(args, ws, rank, local, p, n_acc, acc_seed, skip_empty, 
             b.record(stream)
             torch.cuda.synchronize(dev)
             m2l_ms[lv] = a.elapsed_time(b)
+            m2l_form[lv] = s.m2l_form(lv)
         pot, grad = s.field()
         results[name] = dict(ms=ms, step_ms=step_ms, launches=launches, stages=stages,
-                             m2l_ms=m2l_ms, pot=pot, grad=grad, clocks=clk.summary(),
+                             m2l_ms=m2l_ms, m2l_form=m2l_form, pot=pot, grad=grad, clocks=clk.summary(),
                              coef_bytes=s.coefficient_storage(0)[1])
         if name == "fp64":
             s.close()
@@ -830,9 +853,9 @@ def single_solve_section(args, ws, rank, local, p, n_acc, acc_seed, skip_empty, 
     lv_dom = max(f32["m2l_ms"], key=lambda lv: f32["m2l_ms"][lv])
     if skip_empty:
         pairs[lv_dom] = list4_pairs_at(p.xt, p.x0, p.D, lv_dom, p.xs)
-    fpp = helm_flops_per_pair if helm else lap_flops_per_pair
-    flops = pairs[lv_dom] * fpp(p.order_s[lv_dom])
-    m2l = {"kernel": f"M2L level {lv_dom}, order {p.order_s[lv_dom]}, FP32",
+    form = f32["m2l_form"][lv_dom]
+    flops = pairs[lv_dom] * m2l_flops_per_pair(p.order_s[lv_dom], helm, form)
+    m2l = {"kernel": f"{M2L_KERNELS[form]}: M2L level {lv_dom}, order {p.order_s[lv_dom]}, FP32",
            "ms": f32["m2l_ms"][lv_dom], "algorithmic_flops_per_launch": flops,
            "achieved_tflops": flops / (f32["m2l_ms"][lv_dom] * 1e-3) / 1e12,
            "pairs": pairs[lv_dom],
@@ -884,13 +907,13 @@ def tile_profile_traffic(path=None):
 TILE_HELM_PROFILE = os.path.join(ROOT, "profiles", "k_m2l_tiles_helmholtz_1e5_p14_level4.md")
 
 
-def tile_roofline(local, helm: bool):
-    """The offset-major tile M2L on a dense level at the stream's order 14,
-    FP32: Helmholtz (the stream's dominant kernel) on level 4 of 1e5 points
-    (k = 10, depth 4), or Laplace on level 5 of 3e5 points (depth 5);
-    algorithmic FLOPs of the rotate / coaxial / rotate-back shifts per launch
-    / CUDA-event launch time (L2 flushed before each), against the FP32 FMA
-    peak measured here."""
+def m2l_roofline(local, helm: bool):
+    """The M2L (automatic choice: the column kernel) of a dense level at the
+    stream's order 14, FP32: Helmholtz on level 4 of 1e5 points (k = 10, depth
+    4), or Laplace on level 5 of 3e5 points (depth 5); the FLOPs of the rotate
+    / coaxial / rotate-back shifts that the kernel does per launch / CUDA-event
+    launch time (L2 flushed before each), against the FP32 FMA peak measured
+    here."""
     import torch
 
     from wbfmm_b200 import engine
@@ -905,7 +928,6 @@ def tile_roofline(local, helm: bool):
     flush = torch.empty(256 * 1024 * 1024 // 4, dtype=torch.float32, device=dev)
     cfg = engine.SolverConfig.from_problem(p, engine.FP32)
     with engine.Solver(cfg, stream=stream.cuda_stream) as s:
-        s.set_m2l_kernel(3)
         s.set_sources(p.xs).set_strengths(p.q).set_targets(p.xt).run()
         times = []
         for i in range(6):
@@ -918,15 +940,15 @@ def tile_roofline(local, helm: bool):
             torch.cuda.synchronize(dev)
             if i:
                 times.append(a.elapsed_time(b))
+        form = s.m2l_form(level)
     ms = float(np.mean(times))
     order = p.order_s[level]
-    fpp = helm_flops_per_pair if helm else lap_flops_per_pair
-    flops = list4_pairs(p.depth)[level] * fpp(order)
+    flops = list4_pairs(p.depth)[level] * m2l_flops_per_pair(order, helm, form)
     achieved = flops / (ms * 1e-3) / 1e12
-    prof = TILE_HELM_PROFILE if helm else TILE_PROFILE
+    prof = COLS_HELM_PROFILE if helm else COLS_PROFILE
     name = "Helmholtz, k = 10" if helm else "Laplace"
     return {"bound": "simt",
-            "kernel": f"k_m2l_tiles<float, {'Helmholtz' if helm else 'Laplace'}>: M2L of level "
+            "kernel": f"{M2L_KERNELS[form]}<float, {'Helmholtz' if helm else 'Laplace'}>: M2L of level "
                       f"{level}, order {order}, {n:,} points ({name}), depth {p.depth}",
             "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
             "peak_source": "FP32 FMA throughput measured live (wbfmm_b200_fp32_fma_peak)",
@@ -1066,9 +1088,9 @@ def our_arm(args, ws, rank, local):
                                     label, min(args.steps, 5))
         for k in ("fp32", "fp64"):
             cube[k].pop("step_ms", None)
-    roofline = tile_roofline(local, helm=True)
+    roofline = m2l_roofline(local, helm=True)
     roofline_p2p = p2p_roofline(local)
-    roofline_m2l_laplace = tile_roofline(local, helm=False)
+    roofline_m2l_laplace = m2l_roofline(local, helm=False)
     cpu = None
     if rank == 0 and ws == 1 and not args.no_cpu_baseline:
         from oracle.oracle_api import have_reference
