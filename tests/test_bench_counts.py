@@ -77,6 +77,8 @@ def test_flops_per_pair_even_odd(p, helm):
 @pytest.mark.parametrize("path, total", [
     (bench.TILE_PROFILE, 71.904256e6 + 5.196288e6),
     (bench.TILE_HELM_PROFILE, 11.853056e6),
+    (bench.COLS_PROFILE, 40.130816e6 + 31.327744e6),
+    (bench.COLS_HELM_PROFILE, 11.988736e6 + 5.616896e6),
     (bench.P2P_PROFILE, 18.511872e6 + 222.72e3),
 ])
 def test_profile_traffic_parses_committed_summaries(path, total):
