@@ -325,11 +325,11 @@ k_p2p(EvalParams<T> p) {
   constexpr bool F32 = sizeof(T) == 4;
   constexpr int NA = HELM ? 8 : 4;
   // packed terms, except for Helmholtz potential and gradient in CTAs of 128
-  // that share no box, where they are slower (ms one by one / packed: 49 points per leaf 0.741 /
-  // 0.759, 10 per leaf 0.074 / 0.078; in CTAs of 32, 8 per leaf, 0.324 / 0.284;
-  // 64 shared leaves of 625 points 3.60 / 3.02;
-  // the potential alone, 49 per leaf, 0.547 / 0.510; Laplace, 49 per leaf,
-  // potential and gradient 0.333 / 0.314, the potential alone 0.261 / 0.251)
+  // that share no box, where they are slower (ms one by one / packed: 49 points
+  // per leaf 0.741 / 0.759, 10 per leaf 0.074 / 0.078; in CTAs of 32, 8 per leaf,
+  // 0.324 / 0.284; 64 shared leaves of 625 points 3.60 / 3.02; the potential
+  // alone, 49 per leaf, 0.547 / 0.510; Laplace, 49 per leaf, potential and
+  // gradient 0.333 / 0.314, the potential alone 0.261 / 0.251)
   constexpr bool PACK = F32 && !DIP && !(HELM && POT && GRAD && NT == 128 && !SHARE);
   __shared__ P2PTile<T, HELM, NT> tl;
   __shared__ uint32_t s_st[27], s_pref[28];
